@@ -170,7 +170,6 @@ struct cfdx_lbm {
     float* ns = nullptr;
     float* macro_scratch = nullptr; // 4*N floats, lazily allocated
     double* reduce_partials = nullptr;
-    double* reduce_out = nullptr;
     double* host_reduce = nullptr; // pinned
     int reduce_blocks = 0;
     cudaStream_t stream = nullptr;
@@ -481,11 +480,19 @@ void ensure_reduce(cfdx_lbm* h) {
     int sms = 0;
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->cfg.device), "device attribute");
     const long long rows = static_cast<long long>(h->cfg.ny * h->cfg.nz);
-    h->reduce_blocks = static_cast<int>(std::max(1LL, std::min<long long>(4LL * sms, rows)));
-    h->reduce_partials = static_cast<double*>(
-        device_alloc(sizeof(double) * kReduceFields * static_cast<std::size_t>(h->reduce_blocks), "reduction scratch"));
-    h->reduce_out = static_cast<double*>(device_alloc(sizeof(double) * kReduceFields, "reduction output"));
-    check_cuda(cudaMallocHost(&h->host_reduce, sizeof(double) * kReduceFields), "cudaMallocHost");
+    const long long per_block = reduce_block(h->cfg.nx).y;
+    h->reduce_blocks =
+        static_cast<int>(std::max(1LL, std::min<long long>(4LL * sms, (rows + per_block - 1) / per_block)));
+    // Pinned: the kernel's last block writes the sums straight to the host.
+    if (!h->host_reduce) check_cuda(cudaMallocHost(&h->host_reduce, sizeof(double) * kReduceFields), "cudaMallocHost");
+    // One row of partial sums per block, and one that holds the counter of finished blocks.
+    const std::size_t bytes = sizeof(double) * kReduceFields * (static_cast<std::size_t>(h->reduce_blocks) + 1U);
+    auto* p = static_cast<double*>(device_alloc(bytes, "reduction scratch"));
+    if (const cudaError_t e = cudaMemsetAsync(p, 0, bytes, h->stream); e != cudaSuccess) {
+        device_free(p);
+        check_cuda(e, "cudaMemsetAsync (reduction scratch)");
+    }
+    h->reduce_partials = p;
 }
 
 void release_adjoint(cfdx_lbm* h) {
@@ -512,7 +519,6 @@ void release(cfdx_lbm* h) {
     device_free(h->ns);
     device_free(h->macro_scratch);
     device_free(h->reduce_partials);
-    device_free(h->reduce_out);
     release_adjoint(h);
     for (auto& sg : h->step_graph)
         if (sg.exec) cudaGraphExecDestroy(sg.exec);
@@ -539,6 +545,14 @@ dim3 cell_block(long long nx, long long ny, const LaunchShape& s) {
 dim3 cell_grid(long long nx, long long ny, long long nz, dim3 block) {
     return dim3(static_cast<unsigned>((nx + block.x - 1) / block.x), static_cast<unsigned>((ny + block.y - 1) / block.y),
                 static_cast<unsigned>(nz));
+}
+
+dim3 reduce_block(unsigned long long nx) {
+    // the width that leaves the fewest idle threads beside a row's end, the widest of equals
+    unsigned best = 32U;
+    for (unsigned bx = 32U; bx <= 256U; bx *= 2U)
+        if ((nx + bx - 1U) / bx * bx <= (nx + best - 1U) / best * best) best = bx;
+    return dim3(best, 256U / best, 1U);
 }
 
 cudaError_t launch_step(const KernelKey& k, const LbmArgs& a, dim3 g, dim3 b, cudaStream_t s) {
@@ -1454,11 +1468,8 @@ CFDX_API int cfdx_lbm_reduce(cfdx_lbm* h, double* out) {
         checked(h);
         require(out != nullptr, "null output");
         ensure_reduce(h);
-        check_cuda(launch_reduce(h->key, h->args(), h->reduce_partials, h->reduce_blocks, h->reduce_out, h->stream),
+        check_cuda(launch_reduce(h->key, h->args(), h->reduce_partials, h->reduce_blocks, h->host_reduce, h->stream),
                    "reduction kernel");
-        check_cuda(cudaMemcpyAsync(h->host_reduce, h->reduce_out, sizeof(double) * kReduceFields,
-                                   cudaMemcpyDeviceToHost, h->stream),
-                   "cudaMemcpyAsync (reduction)");
         h->d2h += sizeof(double) * kReduceFields;
         h->sync();
         for (int k = 0; k < kReduceFields; ++k) out[k] = h->host_reduce[k];

@@ -59,8 +59,12 @@ cudaError_t launch_init(const KernelKey& k, const LbmArgs& a, const InitSpec& sp
 cudaError_t launch_macro(const KernelKey& k, const LbmArgs& a, void* rho, void* ux, void* uy, void* uz,
                          bool out_f64, dim3 grid, dim3 block, cudaStream_t s);
 cudaError_t launch_logical(const KernelKey& k, const LbmArgs& a, float* out, dim3 grid, dim3 block, cudaStream_t s);
+// partials: (blocks + 1) rows of kReduceFields, the last holding the counter of finished blocks
+// (zero before the first call; the kernel leaves it zero).  out: device-visible host memory.
 cudaError_t launch_reduce(const KernelKey& k, const LbmArgs& a, double* partials, int blocks, double* out,
                           cudaStream_t s);
+// Threads of the reduction: x along a row, y over rows (256 in all).
+dim3 reduce_block(unsigned long long nx);
 cudaError_t launch_step_oop(const KernelKey& k, const LbmArgs& src, const LbmArgs& dst, dim3 grid, dim3 block,
                             cudaStream_t s);
 cudaError_t launch_adjoint_seed(const KernelKey& k, const AdjointArgs& a, dim3 grid, dim3 block, cudaStream_t s);

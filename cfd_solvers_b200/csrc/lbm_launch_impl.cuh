@@ -204,13 +204,12 @@ cudaError_t Launcher<STORAGE>::reduce(const KernelKey& k, const LbmArgs& a, doub
     using S = typename StorageOf<STORAGE>::type;
     return with_lattice(k.q, [&](auto lat) {
         using L = decltype(lat);
+        auto* done = reinterpret_cast<unsigned*>(partials + static_cast<std::size_t>(blocks) * kReduceFields);
+        const dim3 b = reduce_block(a.nx);
         if (k.flags)
-            k_reduce<L, S, true><<<blocks, kReduceThreads, 0, s>>>(a, partials);
+            k_reduce<L, S, true, true><<<blocks, b, 0, s>>>(a, partials, done, out);
         else
-            k_reduce<L, S, false><<<blocks, kReduceThreads, 0, s>>>(a, partials);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        k_reduce_final<<<1, kReduceThreads, 0, s>>>(partials, blocks, out);
+            k_reduce<L, S, false, true><<<blocks, b, 0, s>>>(a, partials, done, out);
         return cudaGetLastError();
     });
 }

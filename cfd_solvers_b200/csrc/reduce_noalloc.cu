@@ -69,9 +69,9 @@ int scratch_address(int device, double** out) {
 template <class S, class L>
 cudaError_t launch(const ReduceView& v, double* partials, unsigned blocks, double* result) {
     if (v.key.flags)
-        k_reduce<L, S, true><<<blocks, kReduceThreads, 0, v.stream>>>(v.args, partials);
+        k_reduce<L, S, true, false><<<blocks, kReduceThreads, 0, v.stream>>>(v.args, partials, nullptr, nullptr);
     else
-        k_reduce<L, S, false><<<blocks, kReduceThreads, 0, v.stream>>>(v.args, partials);
+        k_reduce<L, S, false, false><<<blocks, kReduceThreads, 0, v.stream>>>(v.args, partials, nullptr, nullptr);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_reduce_final<<<1, kReduceThreads, 0, v.stream>>>(partials, static_cast<int>(blocks), result);
