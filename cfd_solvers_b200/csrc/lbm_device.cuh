@@ -1143,6 +1143,23 @@ __device__ __forceinline__ void init_pairs(const LbmArgs& a, u32 n, const Nbr& o
     }
 }
 
+// Zeroes the slots of wall cell n that no fluid cell initialises: it owns slot
+// i at n + c_j and slot j at n, which a fluid neighbour writes when its wall
+// link points here (bit 2p + 1 of the cell at n + c_j, bit 2p of the cell at
+// n + c_i; on a slab, ghost cells count as walls without any link to them).
+// With this k_init writes every slot and needs no memset before it.
+template <class L, class S, int P = 0>
+__device__ __forceinline__ void init_wall_pairs(const LbmArgs& a, u32 n, const Nbr& o) {
+    if constexpr (P < L::PAIRS) {
+        constexpr int i = 2 * P + 1, j = i + 1;
+        using T = typename S::T;
+        const u32 nj = n + nbr_off<L, j>(o), ni = n + nbr_off<L, i>(o);
+        if (!((a.wall_mask[nj] >> (2 * P + 1)) & 1U)) static_cast<T*>(a.fd[i])[nj] = T(0);
+        if (!((a.wall_mask[ni] >> (2 * P)) & 1U)) static_cast<T*>(a.fd[j])[n] = T(0);
+        init_wall_pairs<L, S, P + 1>(a, n, o);
+    }
+}
+
 template <class L, class S, bool FLAGS>
 __global__ void __launch_bounds__(128) k_init(const __grid_constant__ LbmArgs a, const InitSpec s) {
     using R = typename S::R;
@@ -1155,7 +1172,11 @@ __global__ void __launch_bounds__(128) k_init(const __grid_constant__ LbmArgs a,
     const Nbr o = make_nbr(a, x, y, z);
     if constexpr (FLAGS) {
         const std::uint8_t flag = a.flags[n];
-        if (flag & kFlagTypeMask) return;
+        if (flag & kFlagTypeMask) {
+            static_cast<typename S::T*>(a.fd[0])[n] = typename S::T(0);
+            init_wall_pairs<L, S>(a, n, o);
+            return;
+        }
         if (flag & kFlagNearWall) walls = a.wall_mask[n];
     }
     R rho, ux, uy, uz;
@@ -1455,13 +1476,16 @@ static __global__ void __launch_bounds__(kReduceThreads) k_reduce_final(const do
 // so that no kernel steps, initialises, reduces or reports them.
 template <class L>
 __global__ void __launch_bounds__(128) k_prepare_flags(const __grid_constant__ LbmArgs a, const std::uint8_t* user,
-                                                       std::uint8_t* out, std::uint32_t* mask, int ghost) {
+                                                       std::uint8_t* out, std::uint32_t* mask, std::uint32_t* moving,
+                                                       int ghost) {
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z = blockIdx.z;
     if (x >= a.nx || y >= a.ny) return;
     const u32 n = (z * a.ny + y) * a.nx + x;
-    const std::uint8_t t = user[n] & kFlagTypeMask;
+    const std::uint8_t raw = user[n];
+    if (raw >= 2) *moving = 1U; // every writer stores the same value
+    const std::uint8_t t = raw & kFlagTypeMask;
     if (t != 0 || (ghost && (z == 0 || z == a.nz - 1U))) {
         out[n] = t != 0 ? t : std::uint8_t(1);
         mask[n] = 0U;

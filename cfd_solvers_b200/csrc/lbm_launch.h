@@ -79,7 +79,8 @@ cudaError_t select_near_cells(const std::uint8_t* flags, std::uint32_t cells, st
                               std::uint32_t* count, void* temp, std::size_t* temp_bytes, cudaStream_t s);
 
 // ghost: planes 0 and nz-1 are a z-slab's ghost planes (k_prepare_flags).
+// *moving (zeroed by the caller) is set when some flag is a moving-wall id.
 cudaError_t launch_prepare_flags(int q, const LbmArgs& a, const std::uint8_t* user, std::uint8_t* out,
-                                 std::uint32_t* mask, bool ghost, dim3 grid, dim3 block, cudaStream_t s);
+                                 std::uint32_t* mask, std::uint32_t* moving, bool ghost, dim3 grid, dim3 block, cudaStream_t s);
 
 } // namespace cfdx
