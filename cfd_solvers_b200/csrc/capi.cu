@@ -272,6 +272,7 @@ struct cfdx_lbm {
         std::uint32_t interval = 0;
         std::uint32_t sub = 0;  // sub-checkpoint interval of the reverse sweep (0: one level)
         bool ready = false;     // a forward pass has run and nothing has changed since
+        bool kept = false;      // the frames hold the forward's states of the last segment
         void* checkpoints = nullptr;
         std::size_t checkpoint_bytes = 0;
         void* frames = nullptr;
@@ -1218,34 +1219,6 @@ std::uint64_t step_graphs(cfdx_lbm* h, const LbmArgs& a, dim3 g, dim3 b, std::ui
     return run * kGraphSteps;
 }
 
-// Enqueues `launches` (returning the first launch error) on the handle's stream,
-// inside one captured CUDA graph when the stream is not already being captured:
-// the adjoint's segments are a hundred-odd dependent launches each, and a graph
-// shortens the gaps between them.  A capture is always ended before an error
-// is reported, so the stream never stays in capture mode.
-extern "C++" template <class F> void enqueue_captured(cfdx_lbm* h, const char* what, F&& launches) {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        check_cuda(launches(), what);
-        return;
-    }
-    check_cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-    const cudaError_t launched = launches();
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ended = cudaStreamEndCapture(h->stream, &graph);
-    cudaGraphExec_t exec = nullptr;
-    const cudaError_t made =
-        launched == cudaSuccess && ended == cudaSuccess ? cudaGraphInstantiate(&exec, graph, 0) : cudaSuccess;
-    if (graph) cudaGraphDestroy(graph);
-    check_cuda(launched, what);
-    check_cuda(ended, "cudaStreamEndCapture");
-    check_cuda(made, "cudaGraphInstantiate");
-    const cudaError_t e = cudaGraphLaunch(exec, h->stream);
-    cudaGraphExecDestroy(exec);
-    check_cuda(e, "cudaGraphLaunch");
-}
-
 } // namespace
 
 CFDX_API int cfdx_lbm_step(cfdx_lbm* h, std::uint64_t count) {
@@ -1849,6 +1822,17 @@ void adjoint_reserve(cfdx_lbm* h, std::uint64_t steps, std::uint32_t interval, s
     }
 }
 
+// Segments of the pass: checkpoints lie `interval` steps apart, counted from the
+// last step, so the first segment takes the remainder and the last one, whose
+// states the forward pass leaves in the frames, is as long as any.
+std::uint64_t segment_count(const cfdx_lbm::Adjoint& A) { return (A.steps + A.interval - 1U) / A.interval; }
+std::uint64_t segment_start(const cfdx_lbm::Adjoint& A, std::uint64_t s) {
+    return s == 0U ? 0U : A.steps - (segment_count(A) - s) * A.interval;
+}
+std::uint64_t segment_length(const cfdx_lbm::Adjoint& A, std::uint64_t s) {
+    return (s + 1U == segment_count(A) ? A.steps : segment_start(A, s + 1U)) - segment_start(A, s);
+}
+
 // One level: state k of segment `segment` (0: its checkpoint).
 void* adjoint_frame(cfdx_lbm* h, std::uint64_t segment, std::uint64_t k) {
     char* base = k == 0U ? static_cast<char*>(h->adj.checkpoints) + segment * h->f_bytes
@@ -1863,6 +1847,17 @@ void* adjoint_subcheckpoint(cfdx_lbm* h, std::uint64_t j) {
 }
 void* adjoint_subframe(cfdx_lbm* h, std::uint64_t nsub, std::uint64_t r) {
     return static_cast<char*>(h->adj.frames) + (nsub - 1U + r - 1U) * h->f_bytes;
+}
+// Where the first pass over a segment of `len` steps leaves its state k (0 < k < len): every
+// state with one level; with two, the sub-checkpoints, the states inside the last sub-segment,
+// and the others in two scratch frames.
+void* adjoint_state(cfdx_lbm* h, std::uint64_t segment, std::uint64_t len, std::uint64_t k) {
+    const std::uint64_t m = h->adj.sub;
+    if (!two_level(m, len)) return adjoint_frame(h, segment, k);
+    if (k % m == 0U) return adjoint_subcheckpoint(h, k / m);
+    const std::uint64_t nsub_full = (std::min<std::uint64_t>(h->adj.interval, h->adj.steps) + m - 1U) / m;
+    const std::uint64_t k0 = (len - 1U) / m * m; // start of the last sub-segment
+    return adjoint_subframe(h, nsub_full, k > k0 ? k - k0 : 1U + (k & 1U));
 }
 
 } // namespace
@@ -1895,22 +1890,29 @@ CFDX_API int cfdx_lbm_adjoint_forward(cfdx_lbm* h, std::uint64_t steps, std::uin
         // state bit for bit.  Checkpoints and frames all keep the layout of
         // parity P0 (gather with P0's tables, scatter with P0 ^ 1's); the
         // very last step scatters into the live lattice in the layout its
-        // final time step reads.
+        // final time step reads.  The states of the last segment go where the
+        // reverse sweep, which starts there, would recompute them: that segment
+        // is not recomputed, at no more memory (96 steps, interval 64: 31
+        // recompute steps instead of 94; a pass of one segment: none).
         const int es = storage_bytes(h->key.storage);
         const int P0 = static_cast<int>(A.t0 & 1U);
         const std::uint64_t t_end = A.t0 + steps;
         const dim3 g = h->grid(), b = h->block();
         check_cuda(cudaMemcpyAsync(adjoint_frame(h, 0, 0), h->f, h->f_bytes, cudaMemcpyDeviceToDevice, h->stream),
                    "cudaMemcpyAsync (adjoint checkpoint)");
-        const std::uint64_t segments = (steps + interval - 1U) / interval;
+        const std::uint64_t segments = segment_count(A);
         void* work[2] = {adjoint_frame(h, 0, 1), adjoint_frame(h, 0, 2)};
         void* cur = adjoint_frame(h, 0, 0);
         for (std::uint64_t s = 0; s < segments; ++s) {
-            const std::uint64_t len = std::min<std::uint64_t>(interval, steps - s * interval);
+            const std::uint64_t len = segment_length(A, s);
+            const bool last = s + 1U == segments;
             for (std::uint64_t k = 1; k <= len; ++k) {
-                const bool last = s + 1U == segments && k == len;
-                void* dst = last ? h->f : (k == len ? adjoint_frame(h, s + 1U, 0) : work[k & 1U]);
-                const int scatter_parity = last && static_cast<int>(t_end & 1U) != P0 ? P0 : (P0 ^ 1);
+                void* dst = h->f;
+                if (k < len)
+                    dst = last ? adjoint_state(h, s, len, k) : work[k & 1U];
+                else if (!last)
+                    dst = adjoint_frame(h, s + 1U, 0);
+                const int scatter_parity = dst == h->f && static_cast<int>(t_end & 1U) != P0 ? P0 : (P0 ^ 1);
                 LbmArgs src = h->args_at(cur, es, P0);
                 src.round_seed = h->round_seed(h->t);
                 check_cuda(launch_step_oop(h->key, src, h->args_at(dst, es, scatter_parity), g, b, h->stream),
@@ -1919,6 +1921,7 @@ CFDX_API int cfdx_lbm_adjoint_forward(cfdx_lbm* h, std::uint64_t steps, std::uin
                 ++h->t;
             }
         }
+        A.kept = true;
         A.t_end = h->t;
         A.ready = true;
     });
@@ -1984,58 +1987,58 @@ CFDX_API int cfdx_lbm_adjoint_backward(cfdx_lbm* h, const float* g_rho, const fl
         X.f = h->args();
         X.l = h->args_at(A.lam, lam_es, 1);
         check_cuda(launch_adjoint_seed(h->key, X, g, b, h->stream), "adjoint seed kernel");
-        const std::uint64_t segments = (A.steps + A.interval - 1U) / A.interval;
+        const std::uint64_t segments = segment_count(A);
         std::uint64_t parity = 0;
+        const bool kept = A.kept;
+        A.kept = kept && segments == 1U && !two_level(A.sub, segment_length(A, 0)); // else the sweep reuses the frames
+        const int P = static_cast<int>(A.t0 & 1U); // every checkpoint and frame keeps the layout of t0
+        const char* const what = "adjoint segment kernels";
         for (std::uint64_t s = segments; s-- > 0U;) {
-            const std::uint64_t ts = A.t0 + s * A.interval;
-            const std::uint64_t len = std::min<std::uint64_t>(A.interval, A.t0 + A.steps - ts);
-            const int P = static_cast<int>(A.t0 & 1U); // every checkpoint and frame keeps the layout of t0
+            const std::uint64_t ts = A.t0 + segment_start(A, s);
+            const std::uint64_t len = segment_length(A, s);
+            const bool have = kept && s + 1U == segments; // the forward pass left this segment's states
             // Recompute step from state `src` (time step ts + k - 1 of the forward) into `dst`.
-            const auto recompute = [&](void* src, void* dst, std::uint64_t k) -> cudaError_t {
+            const auto recompute = [&](void* src, void* dst, std::uint64_t k) {
                 LbmArgs a = h->args_at(src, es, P);
                 a.round_seed = h->round_seed(ts + k - 1U); // the forward's step at this time
-                return launch_step_oop(h->key, a, h->args_at(dst, es, P ^ 1), g, b, h->stream);
+                check_cuda(launch_step_oop(h->key, a, h->args_at(dst, es, P ^ 1), g, b, h->stream), what);
             };
             // Adjoint step k of the segment (reading its incoming state, the state k - 1).
-            const auto adjoint = [&](void* state) -> cudaError_t {
+            const auto adjoint = [&](void* state) {
                 X.f = h->args_at(state, es, P);
                 X.l = h->args_at(A.lam, lam_es, static_cast<int>(parity & 1U));
                 ++parity;
-                return launch_adjoint_step(h->key, X, g, b, h->stream);
+                check_cuda(launch_adjoint_step(h->key, X, g, b, h->stream), what);
             };
-            // the segment's recompute and adjoint steps as one graph
-            enqueue_captured(h, "adjoint segment kernels", [&]() -> cudaError_t {
-                cudaError_t e = cudaSuccess;
-                if (!two_level(A.sub, len)) {
-                    for (std::uint64_t k = 1; k < len && e == cudaSuccess; ++k)
-                        e = recompute(adjoint_frame(h, s, k - 1U), adjoint_frame(h, s, k), k);
-                    for (std::uint64_t k = len; k >= 1U && e == cudaSuccess; --k) e = adjoint(adjoint_frame(h, s, k - 1U));
-                    return e;
-                }
-                // Two levels: first the sub-checkpoints (every m-th state, the
-                // others in two scratch frames), then each sub-segment from the
-                // last: its states from its sub-checkpoint, then its adjoint steps.
-                const std::uint64_t m = A.sub, nsub = (len + m - 1U) / m;
-                const std::uint64_t nsub_full = (std::min<std::uint64_t>(A.interval, A.steps) + m - 1U) / m;
-                const auto start = [&](std::uint64_t j) {
-                    return j == 0U ? adjoint_frame(h, s, 0) : adjoint_subcheckpoint(h, j);
+            if (!two_level(A.sub, len)) {
+                for (std::uint64_t k = 1; k < len && !have; ++k)
+                    recompute(adjoint_frame(h, s, k - 1U), adjoint_frame(h, s, k), k);
+                for (std::uint64_t k = len; k >= 1U; --k) adjoint(adjoint_frame(h, s, k - 1U));
+                continue;
+            }
+            // Two levels: first the sub-checkpoints and the last sub-segment's
+            // states (the others in two scratch frames), then each sub-segment
+            // from the last: its states from its sub-checkpoint (the last one's
+            // are there), then its adjoint steps.
+            const std::uint64_t m = A.sub, nsub = (len + m - 1U) / m;
+            const std::uint64_t nsub_full = (std::min<std::uint64_t>(A.interval, A.steps) + m - 1U) / m;
+            const auto start = [&](std::uint64_t j) {
+                return j == 0U ? adjoint_frame(h, s, 0) : adjoint_subcheckpoint(h, j);
+            };
+            void* cur = start(0);
+            for (std::uint64_t k = 1; k < len && !have; ++k) {
+                void* dst = adjoint_state(h, s, len, k);
+                recompute(cur, dst, k);
+                cur = dst;
+            }
+            for (std::uint64_t j = nsub; j-- > 0U;) {
+                const std::uint64_t k0 = j * m, kend = std::min<std::uint64_t>(k0 + m, len);
+                const auto state = [&](std::uint64_t k) {
+                    return k == k0 ? start(j) : adjoint_subframe(h, nsub_full, k - k0);
                 };
-                void* cur = start(0);
-                for (std::uint64_t k = 1; k <= (nsub - 1U) * m && e == cudaSuccess; ++k) {
-                    void* dst = k % m == 0U ? adjoint_subcheckpoint(h, k / m) : adjoint_subframe(h, nsub_full, 1U + (k & 1U));
-                    e = recompute(cur, dst, k);
-                    cur = dst;
-                }
-                for (std::uint64_t j = nsub; j-- > 0U && e == cudaSuccess;) {
-                    const std::uint64_t k0 = j * m, kend = std::min<std::uint64_t>(k0 + m, len);
-                    const auto state = [&](std::uint64_t k) {
-                        return k == k0 ? start(j) : adjoint_subframe(h, nsub_full, k - k0);
-                    };
-                    for (std::uint64_t k = k0 + 1U; k < kend && e == cudaSuccess; ++k) e = recompute(state(k - 1U), state(k), k);
-                    for (std::uint64_t k = kend; k > k0 && e == cudaSuccess; --k) e = adjoint(state(k - 1U));
-                }
-                return e;
-            });
+                for (std::uint64_t k = k0 + 1U; k < kend && j + 1U < nsub; ++k) recompute(state(k - 1U), state(k), k);
+                for (std::uint64_t k = kend; k > k0; --k) adjoint(state(k - 1U));
+            }
         }
         check_cuda(launch_sum_partials(A.tau_partials, blocks, A.tau_out, h->stream), "adjoint tau reduction");
         if (grad_ns) {

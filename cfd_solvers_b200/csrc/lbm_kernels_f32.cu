@@ -10,7 +10,7 @@ namespace cfdx {
 
 // The FP64 partial-sum kernel of the adjoint does not depend on the storage type.
 cudaError_t launch_sum_partials(const double* partials, std::size_t count, double* out, cudaStream_t s) {
-    k_sum_partials<<<1, 256, 0, s>>>(partials, count, out);
+    k_sum_partials<<<1, kSumThreads, 0, s>>>(partials, count, out);
     return cudaGetLastError();
 }
 

@@ -275,3 +275,36 @@ def test_autograd_two_level_recompute_same_gradients(engine):
             (0.5 * ((u - target) ** 2).sum()).backward()
             grads.append(ns_t.grad.cpu().numpy())
     assert np.array_equal(grads[0], grads[1])
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s"])
+@pytest.mark.parametrize("steps, interval, sub", [(1, 1, 0), (5, 1, 0), (7, 7, 0), (7, 64, 0), (10, 4, 0), (12, 4, 0),
+                                                  (13, 8, 2), (16, 8, 3), (9, 16, 4), (25, 12, 5), (24, 12, 11)])
+def test_adjoint_states_kept_by_the_forward(engine, storage, steps, interval, sub):
+    """The reverse sweep takes the last segment's states from the forward pass; gradients equal those
+    of a plan that keeps every state (one segment) bit for bit, and a second sweep's, whatever
+    remainder the first segment gets and whichever sub-checkpoints the last one holds."""
+    cs = engine
+    shape = (12, 10, 9)
+    n = 12 * 10 * 9
+    rng = np.random.default_rng(8)
+    ns = rng.uniform(0, 0.2, n).astype(np.float32)
+    seeds = [rng.normal(size=n).astype(np.float32) for _ in range(3)]
+    walls = np.zeros(shape[::-1], np.uint8)
+    walls[:, 0], walls[:, -1] = 1, 1
+    got = []
+    for plan in ((steps, 0), (interval, sub)):
+        cfg = cs.InPlaceLbmConfig(nx=shape[0], ny=shape[1], nz=shape[2], tau=0.7, collision="trt", storage=storage,
+                                  acceleration_x=1e-5)
+        with cs.EsotericPullCudaSolver(cfg) as s:
+            s.set_flags(walls.reshape(-1))
+            s.set_solid_fraction(ns)
+            s.initialize_taylor_green(0.04)
+            s.step(1)  # an odd start
+            s.adjoint_forward(steps, *plan)
+            got.append(s.adjoint_backward(*seeds))
+            got.append(s.adjoint_backward(*seeds))
+            got.append((s.logical_populations(), 0.0))
+    for k in range(3):
+        assert np.array_equal(got[k][0], got[k + 3][0]) and got[k][1] == got[k + 3][1]
+    assert np.array_equal(got[0][0], got[1][0]) and got[0][1] == got[1][1]

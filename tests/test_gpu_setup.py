@@ -37,7 +37,7 @@ def random_flags(shape, seed):
 
 @pytest.mark.parametrize("lattice", ["d3q19", "d3q27"])
 @pytest.mark.parametrize("storage, typestr", [("fp32", "<f4"), ("fp16s", "<f2"), ("fp64", "<f8")])
-@pytest.mark.parametrize("shape", [(1, 1, 1), (5, 7, 3), (33, 9, 10)], ids=str)
+@pytest.mark.parametrize("shape", [(2, 2, 2), (5, 7, 3), (33, 9, 10)], ids=str)
 def test_init_writes_every_slot(engine, lattice, storage, typestr, shape):
     import torch
 
@@ -110,14 +110,14 @@ def test_moving_walls_are_found_on_the_device(engine, where, value, moving):
 
 
 @pytest.mark.parametrize("storage", ["fp32", "fp16s", "fp64"])
-@pytest.mark.parametrize("shape", [(1, 1, 1), (31, 3, 2), (33, 70, 40), (64, 1, 700), (257, 9, 300)], ids=str)
+@pytest.mark.parametrize("shape", [(2, 2, 2), (31, 3, 2), (33, 70, 40), (64, 2, 700), (257, 9, 300)], ids=str)
 def test_sums_equal_the_fields_sums(engine, storage, shape):
     """Mass, momentum and kinetic energy against FP64 sums of the reported fields: FP64 additions in
     another order differ by at most (cells) ulps of the sum of magnitudes, far inside 1e-10."""
     cs = engine
     nx, ny, nz = shape
     with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=nx, ny=ny, nz=nz, storage=storage)) as s:
-        if nx > 1:
+        if nx > 2:
             s.set_flags(random_flags((nz, ny, nx), 2))
         s.initialize_taylor_green(0.05)
         s.step(2)
