@@ -425,7 +425,19 @@ struct cfdx_lbm {
         }
         return dim3(static_cast<unsigned>(bx), static_cast<unsigned>(by), 1U);
     }
-    dim3 block() const { return cell_block(static_cast<long long>(cfg.nx), static_cast<long long>(cfg.ny), shape); }
+    // FP16 storage: one warp along x in each of four rows.  Its one-cell kernels
+    // are bound by issue slots and resident warps, not by bandwidth, so the
+    // idle warps of a 128-wide block past a row's end, and the wait of its warps
+    // for the one at a wall, cost time (B200: D3Q27 gray adjoint 160^3, 32 steps
+    // 15.8 ms against 18.6 with 128 x 1; D3Q19 LES cavity 151x160x160 90.8 against
+    // 97.5 us; D3Q27 256^3 equal).  FP32 and FP64 kernels are bound by HBM and
+    // keep the wide rows (301x155x133: 178 us, 186 with 32 x 4).
+    dim3 block() const {
+        LaunchShape s = shape;
+        if (key.storage == kStoreF16S && (s.block_x <= 0 || s.block_y <= 0))
+            s = LaunchShape{32, static_cast<int>(std::min<std::size_t>(4U, cfg.ny))};
+        return cell_block(static_cast<long long>(cfg.nx), static_cast<long long>(cfg.ny), s);
+    }
     dim3 grid() const {
         return cell_grid(static_cast<long long>(cfg.nx), static_cast<long long>(cfg.ny),
                          static_cast<long long>(cfg.nz), block());
