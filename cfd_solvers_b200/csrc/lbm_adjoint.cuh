@@ -257,6 +257,7 @@ template <class L, class S, bool FLAGS, bool GRAY>
 __global__ void __launch_bounds__(128, oop_min_blocks<L, S, GRAY>()) k_step_oop(const __grid_constant__ LbmArgs f,
                                                                           const __grid_constant__ LbmArgs s) {
     using R = typename S::R;
+    dependent_begin();
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z = blockIdx.z;
@@ -347,6 +348,7 @@ template <class L, class S> constexpr int adjoint_min_blocks() {
 template <class L, class S, bool FLAGS>
 __global__ void __launch_bounds__(128, adjoint_min_blocks<L, S>()) k_adjoint_step(const __grid_constant__ AdjointArgs A) {
     using R = typename S::R;
+    dependent_begin();
     using LS = typename AdjointStorage<S>::type;
     const LbmArgs& f = A.f;
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;

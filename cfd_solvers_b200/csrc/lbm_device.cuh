@@ -32,6 +32,17 @@ namespace cfdx {
 
 using u32 = std::uint32_t;
 
+// Programmatic dependent launch.  A lattice kernel launched by launch_dependent
+// starts while the kernel before it drains: every block first lets the next
+// kernel of the stream be scheduled, then waits until the one before has
+// finished and its writes are visible.  Nothing is read or written before the
+// wait, and every thread passes it (an early exit would let this kernel finish
+// before its predecessor, and its successor start too soon).
+__device__ __forceinline__ void dependent_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------- storage traits
 // `delta` storage types hand the kernels the deviation f - w_d from the rest
 // weight instead of f itself; the collision then works in deviation space
@@ -1069,6 +1080,7 @@ template <class S> constexpr int pair_min_blocks() { return sizeof(typename S::T
 template <class L, class S, bool LES, bool FLAGS, bool GRAY, int CPT, bool NARROW>
 __global__ void __launch_bounds__(128, step_min_blocks<L, S, GRAY>()) k_step(const __grid_constant__ LbmArgs a) {
     using R = typename S::R;
+    dependent_begin();
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z0 = a.z_first + blockIdx.z * CPT;
@@ -1217,6 +1229,7 @@ template <class L, class S, bool FLAGS, class OutT, bool NARROW = false>
 __global__ void __launch_bounds__(128) k_macro(const __grid_constant__ LbmArgs a, OutT* rho_out, OutT* ux_out,
                                                OutT* uy_out, OutT* uz_out) {
     using R = typename S::R;
+    dependent_begin();
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z = blockIdx.z;
@@ -1406,6 +1419,7 @@ template <class L, class S, bool FLAGS, bool FUSED>
 __global__ void __launch_bounds__(kReduceThreads) k_reduce(const __grid_constant__ LbmArgs a, double* partials,
                                                            unsigned* done, double* out) {
     using R = typename S::R;
+    dependent_begin();
     double acc[kReduceFields] = {0, 0, 0, 0, 0, 0, 0};
     const u32 rows = a.ny * a.nz;
     for (u32 row = blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += gridDim.x * blockDim.y) {

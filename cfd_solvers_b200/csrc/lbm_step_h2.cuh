@@ -136,6 +136,7 @@ __device__ __forceinline__ void h2_stores(const LbmArgs& a, __half* base, const 
 template <class L, bool LES, bool FLAGS, bool GRAY>
 __global__ void __launch_bounds__(128, LES ? CFDX_H2_MIN_BLOCKS_LES : CFDX_H2_MIN_BLOCKS)
     k_step_h2(const __grid_constant__ LbmArgs a) {
+    dependent_begin();
     H2Ctx c;
     c.x0 = 2U * (blockIdx.x * blockDim.x + threadIdx.x);
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(128, LES ? CFDX_H2_MIN_BLOCKS_LES : CFDX_H2_MI
 // wall-link gather, the moving-wall correction, the collision and the store.
 template <class L, class S, bool LES, bool GRAY>
 __global__ void __launch_bounds__(128, step_min_blocks<L, S>()) k_step_list(const __grid_constant__ LbmArgs a) {
+    dependent_begin();
     const u32 k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.near_count) return;
     const u32 n = a.near_list[k];

@@ -450,6 +450,7 @@ template <class L> constexpr unsigned w2_smem_bytes() {
 // of [a.z_first, a.z_end).
 template <class L, bool LES, bool FLAGS, bool GRAY, bool PIPE>
 __global__ void __launch_bounds__(kW2Threads, w2_min_blocks<L>()) k_step_w2(const __grid_constant__ LbmArgs a) {
+    dependent_begin();
     using Wd = W2Words<L>;
     constexpr int W = Wd::count;
     const u32 x0 = 2U * (blockIdx.x * blockDim.x + threadIdx.x);

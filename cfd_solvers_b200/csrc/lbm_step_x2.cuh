@@ -206,6 +206,7 @@ __device__ __forceinline__ void pair_stores(const LbmArgs& a, typename S::T* bas
 
 template <class L, class S, bool LES, bool FLAGS, bool GRAY>
 __global__ void __launch_bounds__(128, pair_min_blocks<S>()) k_step_x2(const __grid_constant__ LbmArgs a) {
+    dependent_begin();
     using R = typename S::R;
     using T = typename S::T;
     PairCtx c;

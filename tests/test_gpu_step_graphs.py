@@ -90,3 +90,32 @@ def test_cached_graph_follows_changes(engine):
                 run(s, steps, single)
             assert a.time_step() == b.time_step()
             assert np.array_equal(a.logical_populations(), b.logical_populations())
+
+
+@pytest.mark.parametrize("q, storage, variant", [(19, "fp32", 0), (19, "fp32", 2), (27, "fp32", 0), (19, "fp64", 0),
+                                                 (19, "fp16s", 0), (19, "fp16s", 1), (19, "fp16s", 2), (27, "fp16s", 0)])
+def test_overlapping_launches_equal_separate_ones(engine, q, storage, variant):
+    """Each lattice kernel may be scheduled while the one before it drains (programmatic dependent
+    launch): steps, reductions, field reads and setters queued back to back equal the same calls
+    with the stream drained after each, bit for bit."""
+    cs = engine
+    out = []
+    for drain in (False, True):
+        with solver(cs, q, storage, "gray", variant) as s:
+            seen = []
+            for k in range(12):
+                s.step(1 + 9 * (k % 3))
+                if drain:
+                    s.wait()
+                if k % 4 == 1:
+                    seen.append(s.reduce())
+                if k % 4 == 2:
+                    s.refresh_device_macroscopic()
+                    s.device_local_acceleration(clear=True)
+                if k % 4 == 3:
+                    s.set_tau(0.62 + 0.01 * k)
+                if drain:
+                    s.wait()
+            out.append((seen, s.logical_populations()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
