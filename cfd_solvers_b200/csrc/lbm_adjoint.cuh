@@ -250,7 +250,7 @@ __device__ __forceinline__ void block_accumulate(double v, double* partials) {
 #define CFDX_OOP_MIN_BLOCKS_Q19 10
 #endif
 template <class L, class S, bool GRAY> constexpr int oop_min_blocks() {
-    return L::Q == 19 && sizeof(typename S::T) != 8 ? CFDX_OOP_MIN_BLOCKS_Q19 : step_min_blocks<L, S, GRAY>();
+    return L::Q == 19 && sizeof(typename S::T) == 4 ? CFDX_OOP_MIN_BLOCKS_Q19 : step_min_blocks<L, S, GRAY>();
 }
 
 template <class L, class S, bool FLAGS, bool GRAY>

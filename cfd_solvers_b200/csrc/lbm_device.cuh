@@ -485,16 +485,22 @@ __device__ __forceinline__ void scatter(const LbmArgs& a, u32 n, const Nbr& o, c
 }
 
 // ------------------------------------------------------------------ helpers
-// Reciprocals.  rcp: the hardware approximation (__fdividef, within 2 ulp),
-// for relaxation rates, which enter a cell's mass and momentum alike.
+// Reciprocals.  rcp: the hardware approximation (within 1 ulp), for relaxation
+// rates, which enter a cell's mass and momentum alike; flushing, because
+// densities and relaxation times are never subnormal and the other form spends
+// several instructions on scaling.
 // rcp_unbiased, for 1/rho in u = j / rho: the collision returns the momentum
 // rho u, so an error in 1/rho that leans one way (an approximation's does)
 // moves every cell's momentum the same way each step.  One Newton-Raphson step
 // r + r (1 - x r) on the approximation leaves a symmetric error of about half
 // an ulp at the cost of two fused multiply-adds.
-__device__ __forceinline__ float rcp(float x) { return __fdividef(1.0F, x); }
+__device__ __forceinline__ float rcp(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 __device__ __forceinline__ float rcp_unbiased(float x) {
-    const float r = __fdividef(1.0F, x);
+    const float r = rcp(x);
     return fmaf(r, fmaf(-x, r, 1.0F), r);
 }
 __device__ __forceinline__ double rcp_unbiased(double x) { return 1.0 / x; }
@@ -636,7 +642,7 @@ __device__ __forceinline__ R les_tau(const R* s, R rho, R irho, R ux, R uy, R uz
 // 2.3e-7 relative per step against FP64.  What remains is the representation
 // error of the FP32 weights themselves, as in the reference.
 template <class R> struct ClassCoef {
-    R a;  // omega+ w rho          (s'/2 equilibrium term: a * t)
+    R a;  // omega+ w rho / 2      (s'/2 equilibrium term: a * 2t; halving is exact)
     R a0; // omega+ w              (DELTA: subtracted)
     R c;  // omega- w rho          (d'/2 equilibrium term: c * (3 c.u))
     R g1; // 3 (1 - omega+/2) w    (s'/2 force term: g1 * ((3 c.u)(c.F) - u.F))
@@ -645,14 +651,12 @@ template <class R> struct ClassCoef {
 
 template <class L, class R, bool FORCE, bool GRAY, bool DELTA, int P = 0>
 __device__ __forceinline__ void collide_pairs(R* f, const R* s, const R* d, const ClassCoef<R>* cc, R ux3, R uy3,
-                                              R uz3, R ux15, R uy15, R uz15, R fx, R fy, R fz, R base, R uf, R a1,
-                                              R b1, R ns) {
+                                              R uz3, R fx, R fy, R fz, R base2, R uf, R a1, R b1, R ns) {
     if constexpr (P < L::PAIRS) {
         constexpr int i = 2 * P + 1, j = i + 1;
         const ClassCoef<R>& k = cc[weight_class<L>(i)];
-        const R cu3 = cdot<L, i>(ux3, uy3, uz3);     // 3 c.u
-        const R cu15 = cdot<L, i>(ux15, uy15, uz15); // 1.5 c.u
-        const R t = cu3 * cu15 + base;
+        const R cu3 = cdot<L, i>(ux3, uy3, uz3); // 3 c.u
+        const R t = cu3 * cu3 + base2;           // 2 (1 - 1.5 u^2 + 4.5 (c.u)^2)
         R sp = DELTA ? k.a * t + (a1 * s[P] - k.a0) : k.a * t + a1 * s[P];
         R dp = k.c * cu3 + b1 * d[P];
         if constexpr (FORCE) {
@@ -670,8 +674,7 @@ __device__ __forceinline__ void collide_pairs(R* f, const R* s, const R* d, cons
         }
         f[i] = oi;
         f[j] = oj;
-        collide_pairs<L, R, FORCE, GRAY, DELTA, P + 1>(f, s, d, cc, ux3, uy3, uz3, ux15, uy15, uz15, fx, fy, fz, base,
-                                                       uf, a1, b1, ns);
+        collide_pairs<L, R, FORCE, GRAY, DELTA, P + 1>(f, s, d, cc, ux3, uy3, uz3, fx, fy, fz, base2, uf, a1, b1, ns);
     }
 }
 
@@ -697,7 +700,7 @@ __device__ __forceinline__ void class_coefficients(ClassCoef<R>* cc, R rho, R om
         const R w = R(L::w(class_rep(k))) * scale[k];
         const R wr = w * rho;
         cc[k].a0 = omega * w;
-        cc[k].a = omega * wr;
+        cc[k].a = (R(0.5) * omega) * wr;
         cc[k].c = omega_m * wr;
         cc[k].g1 = R(3) * gp * w;
         cc[k].g2 = R(3) * gm * w;
@@ -746,9 +749,8 @@ __device__ __forceinline__ void collide(const LbmArgs& a, u32 n, R* f) {
     ClassCoef<R> cc[4];
     const R unit[4] = {R(1), R(1), R(1), R(1)};
     class_coefficients<L, R>(cc, rho, omega, omega_m, gp, gm, unit);
-    collide_pairs<L, R, FORCE, GRAY, DELTA>(f, s, d, cc, R(3) * ux, R(3) * uy, R(3) * uz, R(1.5) * ux, R(1.5) * uy,
-                                            R(1.5) * uz, fx, fy, fz, base, uf, R(0.5) * (R(1) - omega),
-                                            R(0.5) * (R(1) - omega_m), ns);
+    collide_pairs<L, R, FORCE, GRAY, DELTA>(f, s, d, cc, R(3) * ux, R(3) * uy, R(3) * uz, fx, fy, fz, R(2) * base, uf,
+                                            R(0.5) * (R(1) - omega), R(0.5) * (R(1) - omega_m), ns);
 }
 
 // --------------------------------------------------- FP16 scaled collision
@@ -855,31 +857,37 @@ template <class L, int K, int A, int B> struct CoefSecond {
         return weight_class<L>(i) != K ? 0 : comp(i, A) * comp(i, B);
     }
 };
-template <class L, int K, int A, class V> __device__ __forceinline__ V class_sum(const V* v) {
-    return v_csum<CoefFirst<L, K, A>, 0, L::PAIRS>(v);
+template <class Coef, int E> constexpr bool v_any() {
+    for (int p = 0; p < E; ++p)
+        if (Coef::at(p) != 0) return true;
+    return false;
 }
-template <class L, int K, int A, int B, class V> __device__ __forceinline__ V class_sum2(const V* v) {
-    return v_csum<CoefSecond<L, K, A, B>, 0, L::PAIRS>(v);
-}
-// sum_k sum_k-class(v) / s_k over the weight classes 1..K, as a multiply-add chain.
-template <class L, int A, class V> __device__ __forceinline__ V scaled_moment(const V* v, const float* inv, V init) {
-    V r = v_fma(class_sum<L, 1, A>(v), v_splat<V>(inv[1]), init);
-    r = v_fma(class_sum<L, 2, A>(v), v_splat<V>(inv[2]), r);
-    if constexpr (L::Q == 27) r = v_fma(class_sum<L, 3, A>(v), v_splat<V>(inv[3]), r);
+// Sum over the weight classes in storage units of class 2: sum_k (s_2 / s_k)
+// sum_k-class(v), with r1 = s_2 / s_1 and r3 = s_2 / s_3 (exact for the default
+// power-of-two scales).  One multiply-add per class beyond the second; classes
+// without a term (c_a c_b = 0 for the axis pairs when a != b) cost nothing.
+template <class Coef1, class Coef2, class Coef3, class L, class V>
+__device__ __forceinline__ V class_blend(const V* v, float r1, float r3) {
+    V r = v_csum<Coef2, 0, L::PAIRS>(v);
+    if constexpr (v_any<Coef1, L::PAIRS>()) r = v_fma(v_csum<Coef1, 0, L::PAIRS>(v), v_splat<V>(r1), r);
+    if constexpr (L::Q == 27) r = v_fma(v_csum<Coef3, 0, L::PAIRS>(v), v_splat<V>(r3), r);
     return r;
 }
-template <class L, int A, int B, class V>
-__device__ __forceinline__ V scaled_moment2(const V* v, const float* inv, V init) {
-    V r = v_fma(class_sum2<L, 1, A, B>(v), v_splat<V>(inv[1]), init);
-    r = v_fma(class_sum2<L, 2, A, B>(v), v_splat<V>(inv[2]), r);
-    if constexpr (L::Q == 27) r = v_fma(class_sum2<L, 3, A, B>(v), v_splat<V>(inv[3]), r);
-    return r;
+template <class L, int A, class V> __device__ __forceinline__ V blend1(const V* v, float r1, float r3) {
+    return class_blend<CoefFirst<L, 1, A>, CoefFirst<L, 2, A>, CoefFirst<L, 3, A>, L>(v, r1, r3);
+}
+template <class L, int A, int B, class V> __device__ __forceinline__ V blend2(const V* v, float r1, float r3) {
+    return class_blend<CoefSecond<L, 1, A, B>, CoefSecond<L, 2, A, B>, CoefSecond<L, 3, A, B>, L>(v, r1, r3);
 }
 
 // sqrt for the Smagorinsky rate: hardware reciprocal square root (2 ulp);
 // the eddy viscosity needs no correctly rounded square root, and FP16
 // storage rounding is far larger.  x >= 0; x = 0 gives 0.
-__device__ __forceinline__ float les_sqrt(float x) { return __fmul_rn(x, rsqrtf(fmaxf(x, 1.0e-30F))); }
+__device__ __forceinline__ float les_sqrt(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(x, 1.0e-30F)));
+    return __fmul_rn(x, r);
+}
 
 // n: the first cell of V's lanes (lane k is cell n + k).
 template <class L, bool LES, bool GRAY, bool FORCE, class V>
@@ -898,40 +906,38 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
         inv[k] = a.inv_scale[class_rep(k)];
         scl[k] = a.scale[class_rep(k)];
     }
-    const V rho = v_add(scaled_moment<L, 0>(sh, inv, v_mul(h[0], v_splat<V>(inv[0]))), one);
+    const V inv2 = v_splat<V>(inv[2]);
+    const float r1 = __fmul_rn(inv[1], scl[2]), r3 = L::Q == 27 ? __fmul_rn(inv[K], scl[2]) : 0.0F;
+    const V rho = v_add(v_fma(blend1<L, 0>(sh, r1, r3), inv2, v_mul(h[0], v_splat<V>(inv[0]))), one);
     const V zero = v_splat<V>(-0.0F); // x + (-0) == x for every x
-    const V jx = scaled_moment<L, 1>(dh, inv, zero);
-    const V jy = scaled_moment<L, 2>(dh, inv, zero);
-    const V jz = scaled_moment<L, 3>(dh, inv, zero);
     const V irho = v_map(rho, [](float r, int) { return r > 0.0F ? rcp_unbiased(r) : 0.0F; });
-    V ux = v_mul(jx, irho), uy = v_mul(jy, irho), uz = v_mul(jz, irho);
+    const V irho2 = v_mul(irho, inv2); // 1 / (rho s_2)
+    V ux = v_mul(blend1<L, 1>(dh, r1, r3), irho2), uy = v_mul(blend1<L, 2>(dh, r1, r3), irho2),
+      uz = v_mul(blend1<L, 3>(dh, r1, r3), irho2);
     V ax = zero, ay = zero, az = zero;
     if constexpr (FORCE) {
         ax = v_map(ax, [&](float, int k) { float x, y, z; cell_acceleration<float>(a, n + k, x, y, z); return x; });
         ay = v_map(ay, [&](float, int k) { float x, y, z; cell_acceleration<float>(a, n + k, x, y, z); return y; });
         az = v_map(az, [&](float, int k) { float x, y, z; cell_acceleration<float>(a, n + k, x, y, z); return z; });
-        const V half = v_splat<V>(0.5F);
-        ux = v_fma(ax, half, ux);
-        uy = v_fma(ay, half, uy);
-        uz = v_fma(az, half, uz);
+        const V ahalf = v_splat<V>(0.5F);
+        ux = v_fma(ax, ahalf, ux);
+        uy = v_fma(ay, ahalf, uy);
+        uz = v_fma(az, ahalf, uz);
     }
     V omega, omega_m;
     if constexpr (LES) {
         const V third = v_splat<V>(1.0F / 3.0F);
-        const V sxx = scaled_moment2<L, 1, 1>(sh, inv, third);
-        const V syy = scaled_moment2<L, 2, 2>(sh, inv, third);
-        const V szz = scaled_moment2<L, 3, 3>(sh, inv, third);
-        const V sxy = scaled_moment2<L, 1, 2>(sh, inv, zero);
-        const V sxz = scaled_moment2<L, 1, 3>(sh, inv, zero);
-        const V syz = scaled_moment2<L, 2, 3>(sh, inv, zero);
+        const V sxx = v_fma(blend2<L, 1, 1>(sh, r1, r3), inv2, third);
+        const V syy = v_fma(blend2<L, 2, 2>(sh, r1, r3), inv2, third);
+        const V szz = v_fma(blend2<L, 3, 3>(sh, r1, r3), inv2, third);
         const V nrho = v_mul(rho, v_splat<V>(-1.0F));
         const V pxx = v_fma(nrho, v_fma(ux, ux, third), sxx);
         const V pyy = v_fma(nrho, v_fma(uy, uy, third), syy);
         const V pzz = v_fma(nrho, v_fma(uz, uz, third), szz);
         const V nrux = v_mul(nrho, ux), nruy = v_mul(nrho, uy);
-        const V pxy = v_fma(nrux, uy, sxy);
-        const V pxz = v_fma(nrux, uz, sxz);
-        const V pyz = v_fma(nruy, uz, syz);
+        const V pxy = v_fma(blend2<L, 1, 2>(sh, r1, r3), inv2, v_mul(nrux, uy));
+        const V pxz = v_fma(blend2<L, 1, 3>(sh, r1, r3), inv2, v_mul(nrux, uz));
+        const V pyz = v_fma(blend2<L, 2, 3>(sh, r1, r3), inv2, v_mul(nruy, uz));
         V off = v_mul(pxy, pxy);
         off = v_fma(pxz, pxz, off);
         off = v_fma(pyz, pyz, off);
@@ -953,10 +959,10 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
         omega = v_splat<V>(w);
         omega_m = v_splat<V>(omega_minus_of<float>(a, a.tau_f, w));
     }
-    V base = v_mul(ux, ux);
-    base = v_fma(uy, uy, base);
-    base = v_fma(uz, uz, base);
-    base = v_fma(base, v_splat<V>(-1.5F), one);
+    V base2 = v_mul(ux, ux);
+    base2 = v_fma(uy, uy, base2);
+    base2 = v_fma(uz, uz, base2);
+    base2 = v_fma(base2, v_splat<V>(-3.0F), v_splat<V>(2.0F)); // 2 - 3 u^2
     V fx = zero, fy = zero, fz = zero, nuf = zero;
     if constexpr (FORCE) {
         fx = v_mul(rho, ax);
@@ -967,8 +973,13 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
         uf = v_fma(uz, fz, uf);
         nuf = v_mul(uf, v_splat<V>(-1.0F));
     }
-    const V nhalf = v_splat<V>(-0.5F);
-    const V gp = v_fma(omega, nhalf, one), gm = v_fma(omega_m, nhalf, one);
+    const V half = v_splat<V>(0.5F);
+    const V omegah = v_mul(omega, half);
+    V gp = zero, gm = zero;
+    if constexpr (FORCE) {
+        gp = v_sub(one, omegah);
+        gm = v_fma(omega_m, v_splat<V>(-0.5F), one);
+    }
     V ns = zero, keep = one;
     if constexpr (GRAY) {
         ns = v_map(ns, [&](float, int k) { return a.ns[n + k]; });
@@ -977,19 +988,19 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
     {
         const float w0 = float(L::w(0)) * scl[0];
         const V h0 = h[0];
-        // (1 - omega) h0 + s0 omega w0 (rho base - 1)  [- s0 (1 - omega/2) w0 3 u.F]
-        V o0 = v_fma(v_sub(one, omega), h0, v_mul(v_mul(omega, v_splat<V>(w0)), v_fma(rho, base, v_splat<V>(-1.0F))));
+        // (1 - omega) h0 + s0 (omega/2) w0 (rho (2 - 3 u^2) - 2)  [- s0 (1 - omega/2) w0 3 u.F]
+        V o0 = v_fma(v_sub(one, omega), h0, v_mul(v_mul(omegah, v_splat<V>(w0)), v_fma(rho, base2, v_splat<V>(-2.0F))));
         if constexpr (FORCE) o0 = v_fma(v_mul(gp, v_splat<V>(3.0F * w0)), nuf, o0);
         if constexpr (GRAY) o0 = v_fma(keep, o0, v_mul(ns, h0));
         h[0] = o0;
     }
-    // per weight class: a = omega w rho, a0 = omega w, c = omega- w rho (w includes the storage scale)
+    // per weight class: a = omega w rho / 2, a0 = omega w, c = omega- w rho (w includes the storage scale)
     V ka[4], nka0[4], kc[4], g1[4], g2[4];
 #pragma unroll
     for (int k = 1; k <= K; ++k) {
         const float w = float(L::w(class_rep(k))) * scl[k];
         const V wr = v_mul(rho, v_splat<V>(w));
-        ka[k] = v_mul(omega, wr);
+        ka[k] = v_mul(omegah, wr);
         kc[k] = v_mul(omega_m, wr);
         nka0[k] = v_mul(omega, v_splat<V>(-w));
         if constexpr (FORCE) {
@@ -997,17 +1008,15 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
             g2[k] = v_mul(gm, v_splat<V>(3.0F * w));
         }
     }
-    const V a1 = v_mul(v_sub(one, omega), v_splat<V>(0.5F));
-    const V b1 = v_mul(v_sub(one, omega_m), v_splat<V>(0.5F));
+    const V a1 = v_sub(half, omegah);
+    const V b1 = v_fma(omega_m, v_splat<V>(-0.5F), half);
     const V ux3 = v_mul(ux, v_splat<V>(3.0F)), uy3 = v_mul(uy, v_splat<V>(3.0F)), uz3 = v_mul(uz, v_splat<V>(3.0F));
-    const V ux15 = v_mul(ux, v_splat<V>(1.5F)), uy15 = v_mul(uy, v_splat<V>(1.5F)), uz15 = v_mul(uz, v_splat<V>(1.5F));
     static_for_pairs<L>([&](auto PP) {
         constexpr int p = decltype(PP)::value;
         constexpr int i = 2 * p + 1, j = i + 1;
         constexpr int k = weight_class<L>(i);
         const V cu3 = v_cdot<L, i>(ux3, uy3, uz3);
-        const V cu15 = v_cdot<L, i>(ux15, uy15, uz15);
-        const V t = v_fma(cu3, cu15, base);
+        const V t = v_fma(cu3, cu3, base2); // 2 (1 - 1.5 u^2 + 4.5 (c.u)^2)
         V sp = v_fma(ka[k], t, v_fma(a1, sh[p], nka0[k]));
         V dp = v_fma(kc[k], cu3, v_mul(b1, dh[p]));
         if constexpr (FORCE) {
@@ -1038,12 +1047,15 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
 // uncapped 64-96 registers by 10-55% for FP32 and FP16 storage, and for D3Q19
 // 12 blocks (40 registers) beat 10 once the wall path stopped branching (LES
 // cavity FP16 48.4 vs 46.9, FP32 40.6 vs 40.0; sphere pack within 0.5 %);
+// D3Q27 FP16 runs at 8 blocks (64 registers), where it does not spill: periodic
+// BGK 128^3 49.5 us against 54.6 at 10, 256x128x128 sphere pack 120.4 against
+// 123.2, 256^3 LES cavity 476 against 478.
 // FP64 storage keeps its full register set.  The macros exist for tuning builds.
 #ifndef CFDX_STEP_MIN_BLOCKS_Q19
 #define CFDX_STEP_MIN_BLOCKS_Q19 12
 #endif
 #ifndef CFDX_STEP_MIN_BLOCKS_Q27_F16
-#define CFDX_STEP_MIN_BLOCKS_Q27_F16 10
+#define CFDX_STEP_MIN_BLOCKS_Q27_F16 8
 #endif
 #ifndef CFDX_STEP_MIN_BLOCKS_Q27_F32
 #define CFDX_STEP_MIN_BLOCKS_Q27_F32 8
@@ -1056,21 +1068,23 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
 // 112 (D3Q19 FP32) and 368 (D3Q27 FP16) bytes per thread at the caps above.
 // Measured on B200, gray TRT channel forward step: D3Q27 FP16 256^3 at 8
 // blocks (64 registers) 548 us vs 744 us at 10; D3Q19 FP32 128^3 at 8 blocks
-// 63.7 us vs 65.9 us at 12 (10 blocks, 48 registers, keeps 24 bytes of spill).
+// 63.7 us vs 65.9 us at 12 (10 blocks, 48 registers, keeps 24 bytes of spill);
+// D3Q19 FP16, gray adjoint 128^3 (96 steps) 16.95 ms at 8 blocks, 17.24 at 10.
 #ifndef CFDX_STEP_MIN_BLOCKS_Q19_GRAY
 #define CFDX_STEP_MIN_BLOCKS_Q19_GRAY 10
 #endif
-#ifndef CFDX_STEP_MIN_BLOCKS_Q27_F16_GRAY
-#define CFDX_STEP_MIN_BLOCKS_Q27_F16_GRAY 8
+#ifndef CFDX_STEP_MIN_BLOCKS_F16_GRAY
+#define CFDX_STEP_MIN_BLOCKS_F16_GRAY 8
 #endif
 
 template <class L, class S, bool GRAY = false> constexpr int step_min_blocks() {
     if constexpr (sizeof(typename S::T) == 8) {
         return 1;
     } else if constexpr (L::Q == 19) {
-        return GRAY ? CFDX_STEP_MIN_BLOCKS_Q19_GRAY : CFDX_STEP_MIN_BLOCKS_Q19;
+        if constexpr (GRAY) return sizeof(typename S::T) == 2 ? CFDX_STEP_MIN_BLOCKS_F16_GRAY : CFDX_STEP_MIN_BLOCKS_Q19_GRAY;
+        else return CFDX_STEP_MIN_BLOCKS_Q19;
     } else if constexpr (sizeof(typename S::T) == 2) {
-        return GRAY ? CFDX_STEP_MIN_BLOCKS_Q27_F16_GRAY : CFDX_STEP_MIN_BLOCKS_Q27_F16;
+        return GRAY ? CFDX_STEP_MIN_BLOCKS_F16_GRAY : CFDX_STEP_MIN_BLOCKS_Q27_F16;
     } else {
         return CFDX_STEP_MIN_BLOCKS_Q27_F32;
     }
