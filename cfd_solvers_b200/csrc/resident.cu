@@ -187,8 +187,8 @@ struct Rows {
 
 __device__ __forceinline__ bool rows_of(const ThermalGrid& t, Rows& r) {
     r.x0 = 4U * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (r.x0 >= t.nx) return false;
-    const u32 y = blockIdx.y, z = blockIdx.z;
+    const u32 y = blockIdx.y * blockDim.y + threadIdx.y, z = blockIdx.z;
+    if (r.x0 >= t.nx || y >= t.ny) return false;
     r.c = at(r.x0, y, z, t);
     r.yp = at(r.x0, shp(y, t.ny), z, t);
     r.ym = at(r.x0, shm(y, t.ny), z, t);
@@ -340,8 +340,8 @@ __device__ __forceinline__ Nb q_nb(const QColumn& col, float4 yp, float4 ym, int
 __global__ void __launch_bounds__(128) k_resident_q4z(const float* ux, const float* uy, const float* uz, ThermalGrid t,
                                                       float* q) {
     const u32 x0 = 4U * (blockIdx.x * blockDim.x + threadIdx.x);
-    if (x0 >= t.nx) return;
-    const u32 y = blockIdx.y, z0 = blockIdx.z * kQPlanes;
+    const u32 y = blockIdx.y * blockDim.y + threadIdx.y, z0 = blockIdx.z * kQPlanes;
+    if (x0 >= t.nx || y >= t.ny) return;
     const u32 z_end = min(z0 + kQPlanes, t.nz);
     const u32 yp = shp(y, t.ny), ym = shm(y, t.ny);
     const u32 xl = x0 == 0U ? t.nx - 1U : x0 - 1U, xr = x0 + 4U == t.nx ? 0U : x0 + 4U;
@@ -431,72 +431,116 @@ __device__ __forceinline__ u32 wrap(long long v, u32 extent) {
     return static_cast<u32>(v);
 }
 
-__global__ void __launch_bounds__(128) k_particles(float* st, u32 count, ThermalGrid t, const float* ux,
-                                                   const float* uy, const float* uz, float* ax, float* ay, float* az,
-                                                   float dt, int two_way, float gx, float gy, float gz) {
+// Cell index of a wrapped coordinate p with floor i: in range but for rounding
+// at the upper face and for positions that are not finite or overflowed.
+__device__ __forceinline__ u32 cell_index(long long i, u32 extent) {
+    return i >= 0 && i < static_cast<long long>(extent) ? static_cast<u32>(i) : wrap(i, extent);
+}
+
+// The values at x0 and x0 + 1 of a row.  PAIRS: rows start 8-byte aligned (even
+// nx, aligned fields), so an even x0 below the last takes one 8-byte access.
+template <bool PAIRS> __device__ __forceinline__ float2 row_pair(const float* f, u32 n0, u32 n1, bool joint) {
+    if (PAIRS && joint) return *reinterpret_cast<const float2*>(f + n0);
+    return make_float2(f[n0], f[n1]);
+}
+template <bool PAIRS> __device__ __forceinline__ void add_pair(float* f, u32 n0, u32 n1, bool joint, float a, float b) {
+    if (PAIRS && joint) {
+        atomicAdd(reinterpret_cast<float2*>(f + n0), make_float2(a, b));
+    } else {
+        atomicAdd(f + n0, a);
+        atomicAdd(f + n1, b);
+    }
+}
+
+// Bound by the latency and the sectors of its scattered accesses (24 loads and
+// 24 additions per particle, each lane in a sector of its own).  2^18 particles
+// at random in 192^3 cells: 90.5 us with joint accesses and 32-bit indices, 100.4
+// with a scalar access per corner and 64-bit remainders (B200); more resident
+// blocks (10, 12 per SM) change nothing.
+template <bool PAIRS>
+__global__ void __launch_bounds__(128, 8) k_particles(float* st, u32 count, ThermalGrid t, const float* ux,
+                                                       const float* uy, const float* uz, float* ax, float* ay,
+                                                       float* az, float dt, int two_way, float gx, float gy, float gz) {
     const u32 p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= count) return;
     float px = periodic(st[p], t.nx), py = periodic(st[count + p], t.ny), pz = periodic(st[2U * count + p], t.nz);
-    float vx = st[3U * count + p], vy = st[4U * count + p], vz = st[5U * count + p];
-    const float mass = st[6U * count + p], response = st[7U * count + p];
     // a position that is not finite (an overflowed velocity) samples cell 0 instead of
     // converting inf/NaN to an integer
     const long long x0 = isfinite(px) ? floor_ll(px) : 0, y0 = isfinite(py) ? floor_ll(py) : 0,
                     z0 = isfinite(pz) ? floor_ll(pz) : 0;
     const float tx = __fsub_rn(px, float(x0)), ty = __fsub_rn(py, float(y0)), tz = __fsub_rn(pz, float(z0));
+    const u32 xi = cell_index(x0, t.nx), yi = cell_index(y0, t.ny), zi = cell_index(z0, t.nz);
+    const u32 xn = shp(xi, t.nx), ys[2] = {yi, shp(yi, t.ny)}, zs[2] = {zi, shp(zi, t.nz)};
+    const bool joint = (xi & 1U) == 0U && xn == xi + 1U;
+    const float wx[2] = {__fsub_rn(1.0F, tx), tx}, wy[2] = {__fsub_rn(1.0F, ty), ty}, wz[2] = {__fsub_rn(1.0F, tz), tz};
+    float2 u[4], v[4], w[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) { // rows in (dz, dy) order
+        const u32 row = (zs[r >> 1] * t.ny + ys[r & 1]) * t.nx;
+        u[r] = row_pair<PAIRS>(ux, row + xi, row + xn, joint);
+        v[r] = row_pair<PAIRS>(uy, row + xi, row + xn, joint);
+        w[r] = row_pair<PAIRS>(uz, row + xi, row + xn, joint);
+    }
     float fu = 0.0F, fv = 0.0F, fw = 0.0F;
-    u32 ids[8];
-    float weights[8];
-    int k = 0;
 #pragma unroll
-    for (int dz = 0; dz <= 1; ++dz)
-#pragma unroll
-        for (int dy = 0; dy <= 1; ++dy)
-#pragma unroll
-            for (int dx = 0; dx <= 1; ++dx) {
-                const float wx = dx ? tx : __fsub_rn(1.0F, tx), wy = dy ? ty : __fsub_rn(1.0F, ty),
-                            wz = dz ? tz : __fsub_rn(1.0F, tz);
-                const u32 n = at(wrap(x0 + dx, t.nx), wrap(y0 + dy, t.ny), wrap(z0 + dz, t.nz), t);
-                const float w = __fmul_rn(__fmul_rn(wx, wy), wz);
-                ids[k] = n;
-                weights[k] = w;
-                ++k;
-                fu = __fadd_rn(fu, __fmul_rn(w, ux[n]));
-                fv = __fadd_rn(fv, __fmul_rn(w, uy[n]));
-                fw = __fadd_rn(fw, __fmul_rn(w, uz[n]));
-            }
+    for (int r = 0; r < 4; ++r) {
+        const float a = __fmul_rn(__fmul_rn(wx[0], wy[r & 1]), wz[r >> 1]);
+        const float b = __fmul_rn(__fmul_rn(wx[1], wy[r & 1]), wz[r >> 1]);
+        fu = __fadd_rn(__fadd_rn(fu, __fmul_rn(a, u[r].x)), __fmul_rn(b, u[r].y));
+        fv = __fadd_rn(__fadd_rn(fv, __fmul_rn(a, v[r].x)), __fmul_rn(b, v[r].y));
+        fw = __fadd_rn(__fadd_rn(fw, __fmul_rn(a, w[r].x)), __fmul_rn(b, w[r].y));
+    }
+    float vx = st[3U * count + p], vy = st[4U * count + p], vz = st[5U * count + p];
+    const float mass = st[6U * count + p], response = st[7U * count + p];
     const float dragx = __fdiv_rn(__fmul_rn(mass, __fsub_rn(fu, vx)), response);
     const float dragy = __fdiv_rn(__fmul_rn(mass, __fsub_rn(fv, vy)), response);
     const float dragz = __fdiv_rn(__fmul_rn(mass, __fsub_rn(fw, vz)), response);
     if (two_way) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            atomicAdd(ax + ids[j], __fmul_rn(-dragx, weights[j]));
-            atomicAdd(ay + ids[j], __fmul_rn(-dragy, weights[j]));
-            atomicAdd(az + ids[j], __fmul_rn(-dragz, weights[j]));
+        for (int r = 0; r < 4; ++r) {
+            const u32 row = (zs[r >> 1] * t.ny + ys[r & 1]) * t.nx;
+            const float a = __fmul_rn(__fmul_rn(wx[0], wy[r & 1]), wz[r >> 1]);
+            const float b = __fmul_rn(__fmul_rn(wx[1], wy[r & 1]), wz[r >> 1]);
+            add_pair<PAIRS>(ax, row + xi, row + xn, joint, __fmul_rn(-dragx, a), __fmul_rn(-dragx, b));
+            add_pair<PAIRS>(ay, row + xi, row + xn, joint, __fmul_rn(-dragy, a), __fmul_rn(-dragy, b));
+            add_pair<PAIRS>(az, row + xi, row + xn, joint, __fmul_rn(-dragz, a), __fmul_rn(-dragz, b));
         }
     }
     vx = __fadd_rn(vx, __fmul_rn(dt, __fadd_rn(__fdiv_rn(dragx, mass), gx)));
     vy = __fadd_rn(vy, __fmul_rn(dt, __fadd_rn(__fdiv_rn(dragy, mass), gy)));
     vz = __fadd_rn(vz, __fmul_rn(dt, __fadd_rn(__fdiv_rn(dragz, mass), gz)));
-    px = periodic(__fadd_rn(px, __fmul_rn(dt, vx)), t.nx);
-    py = periodic(__fadd_rn(py, __fmul_rn(dt, vy)), t.ny);
-    pz = periodic(__fadd_rn(pz, __fmul_rn(dt, vz)), t.nz);
-    st[p] = px;
-    st[count + p] = py;
-    st[2U * count + p] = pz;
+    st[p] = periodic(__fadd_rn(px, __fmul_rn(dt, vx)), t.nx);
+    st[count + p] = periodic(__fadd_rn(py, __fmul_rn(dt, vy)), t.ny);
+    st[2U * count + p] = periodic(__fadd_rn(pz, __fmul_rn(dt, vz)), t.nz);
     st[3U * count + p] = vx;
     st[4U * count + p] = vy;
     st[5U * count + p] = vz;
 }
 
 dim3 cell_grid3(const ThermalGrid& t) { return dim3((t.nx + 127U) / 128U, t.ny, t.nz); }
-dim3 quad_grid(const ThermalGrid& t) { return dim3((t.nx / 4U + 127U) / 128U, t.ny, t.nz); }
+// Blocks of the four-cell kernels: 128 threads, as wide along x as leaves the
+// fewest idle past a row's end (192 cells are 48 quads: 16 x 8, all live,
+// where 128 x 1 left 80 of 128 idle), at least 8 quads (128 bytes) wide.
+// 192^3 (B200, us): normals 45 -> 33, tension 40 -> 31, advection 32 -> 27,
+// Q 47 -> 32, curvature 22.6 -> 17.
+dim3 quad_block(const ThermalGrid& t) {
+    const u32 quads = t.nx / 4U;
+    u32 best = 8U;
+    for (u32 bx = 8U; bx <= 128U; bx *= 2U)
+        if ((quads + bx - 1U) / bx * bx <= (quads + best - 1U) / best * best) best = bx;
+    return dim3(best, 128U / best);
+}
+dim3 quad_grid(const ThermalGrid& t, u32 planes = 1U) {
+    const dim3 b = quad_block(t);
+    return dim3((t.nx / 4U + b.x - 1U) / b.x, (t.ny + b.y - 1U) / b.y, (t.nz + planes - 1U) / planes);
+}
 
-bool aligned16(const void* p) { return (reinterpret_cast<std::uintptr_t>(p) & 15U) == 0U; }
+template <class... P> bool aligned(std::uintptr_t bytes, P... fields) {
+    return ((reinterpret_cast<std::uintptr_t>(fields) % bytes == 0U) && ...);
+}
 // The four-cell kernels need whole float4 rows: nx % 4 == 0 and 16-byte aligned fields.
 template <class... P> bool quads(const ThermalGrid& t, P... fields) {
-    return t.nx % 4U == 0U && (aligned16(fields) && ...);
+    return t.nx % 4U == 0U && aligned(16U, fields...);
 }
 
 } // namespace
@@ -514,7 +558,7 @@ cudaError_t launch_fill_half_space_x(float* fill, ThermalGrid t, float interface
 cudaError_t launch_fill_advect(const float* fill, float* out, ThermalGrid t, const float* ux, const float* uy,
                                const float* uz, float dt, cudaStream_t s) {
     if (quads(t, fill, out, ux, uy, uz))
-        k_fill_advect4<<<quad_grid(t), 128, 0, s>>>(fill, out, t, ux, uy, uz, dt);
+        k_fill_advect4<<<quad_grid(t), quad_block(t), 0, s>>>(fill, out, t, ux, uy, uz, dt);
     else
         k_fill_advect<<<cell_grid3(t), 128, 0, s>>>(fill, out, t, ux, uy, uz, dt);
     return cudaGetLastError();
@@ -523,13 +567,13 @@ cudaError_t launch_fill_advect(const float* fill, float* out, ThermalGrid t, con
 cudaError_t launch_fill_geometry(const float* fill, float* geometry, ThermalGrid t, cudaStream_t s) {
     const bool q4 = quads(t, fill, geometry);
     if (q4)
-        k_fill_normals4<<<quad_grid(t), 128, 0, s>>>(fill, geometry, t);
+        k_fill_normals4<<<quad_grid(t), quad_block(t), 0, s>>>(fill, geometry, t);
     else
         k_fill_normals<<<cell_grid3(t), 128, 0, s>>>(fill, geometry, t);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (q4)
-        k_fill_curvature4<<<quad_grid(t), 128, 0, s>>>(geometry, t);
+        k_fill_curvature4<<<quad_grid(t), quad_block(t), 0, s>>>(geometry, t);
     else
         k_fill_curvature<<<cell_grid3(t), 128, 0, s>>>(geometry, t);
     return cudaGetLastError();
@@ -538,7 +582,7 @@ cudaError_t launch_fill_geometry(const float* fill, float* geometry, ThermalGrid
 cudaError_t launch_surface_tension(const float* fill, const float* curvature, ThermalGrid t, float* ax, float* ay,
                                    float* az, float sigma, float density, cudaStream_t s) {
     if (quads(t, fill, curvature, ax, ay, az))
-        k_surface_tension4<<<quad_grid(t), 128, 0, s>>>(fill, curvature, t, ax, ay, az, sigma, density);
+        k_surface_tension4<<<quad_grid(t), quad_block(t), 0, s>>>(fill, curvature, t, ax, ay, az, sigma, density);
     else
         k_surface_tension<<<cell_grid3(t), 128, 0, s>>>(fill, curvature, t, ax, ay, az, sigma, density);
     return cudaGetLastError();
@@ -557,16 +601,17 @@ cudaError_t launch_particles_advance(float* state, std::uint32_t count, ThermalG
                                      const float* uy, const float* uz, float* ax, float* ay, float* az, float dt,
                                      bool two_way, float gx, float gy, float gz, cudaStream_t s) {
     if (count == 0U) return cudaSuccess;
-    k_particles<<<(count + 127U) / 128U, 128, 0, s>>>(state, count, t, ux, uy, uz, ax, ay, az, dt, two_way ? 1 : 0,
-                                                      gx, gy, gz);
+    const bool pairs = t.nx % 2U == 0U && aligned(8U, ux, uy, uz, ax, ay, az);
+    const auto kernel = pairs ? k_particles<true> : k_particles<false>;
+    kernel<<<(count + 127U) / 128U, 128, 0, s>>>(state, count, t, ux, uy, uz, ax, ay, az, dt, two_way ? 1 : 0, gx, gy,
+                                                 gz);
     return cudaGetLastError();
 }
 
 cudaError_t launch_resident_q(const float* ux, const float* uy, const float* uz, ThermalGrid t, float* q,
                               cudaStream_t s) {
     if (quads(t, ux, uy, uz, q))
-        k_resident_q4z<<<dim3((t.nx / 4U + 127U) / 128U, t.ny, (t.nz + kQPlanes - 1U) / kQPlanes), 128, 0, s>>>(
-            ux, uy, uz, t, q);
+        k_resident_q4z<<<quad_grid(t, kQPlanes), quad_block(t), 0, s>>>(ux, uy, uz, t, q);
     else
         k_resident_q<<<cell_grid3(t), 128, 0, s>>>(ux, uy, uz, t, q);
     return cudaGetLastError();
