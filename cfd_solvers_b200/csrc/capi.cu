@@ -220,8 +220,29 @@ struct cfdx_lbm {
     // step kernel: 0 auto, 1 one cell per thread, 2 paired cells, 3 / 4 the
     // wall-aware z-marching FP16 pair kernel with / without its cp.async pipeline
     int variant = 0;
-    std::uint32_t planes = 0; // z-planes per thread of that kernel (0: kDefaultPlanes)
-    static constexpr std::uint32_t kDefaultPlanes = 4; // measured: 4 > 8 > 16 on the 512^3 cavity
+    std::uint32_t planes = 0; // z-planes per thread of that kernel (0: auto_planes)
+    int sms = 0;              // multiprocessors of the device
+    // z-planes per thread of the z-marching pair kernel.  Short marches start
+    // the look-ahead more often (per plane, 512^3 cavity: 1 / 1.003 / 1.018 /
+    // 1.152 at 4 / 3 / 2 / 1 planes; 8 and 16 lose there too), long ones leave a
+    // longer tail: about one block's march on top of its share of the work, at
+    // five resident blocks per SM.  B200, us per step at 4 / 3 / 2 / 1 planes:
+    // LES cavities 512^3 2395 / 2404 / 2437 / 2758, 256^3 329 / 330 / 325 / -, 128^3
+    // 48.9 / 46.7 / 44.4 / 44.2, 64^3 24.3 / 16.2 / 13.5 / 9.8; sphere packs
+    // 512x256x256 686 / 695 / 716 / -, 100x90x80 25.4 / 24.6 / 23.1 / 22.4.
+    std::uint32_t auto_planes() const {
+        const std::size_t across = (cfg.nx / 2U + 31U) / 32U * ((cfg.ny + 3U) / 4U);
+        const std::size_t resident = 5U * static_cast<std::size_t>(std::max(sms, 1));
+        constexpr std::size_t march[5] = {0U, 1152U, 2035U, 3010U, 4000U};
+        std::uint32_t best = 4U;
+        for (std::uint32_t p = 3U; p >= 1U; --p) {
+            const auto cost = [&](std::uint32_t k) {
+                return (across * ((cfg.nz + k - 1U) / k) + resident) * march[k];
+            };
+            if (cost(p) < cost(best)) best = p;
+        }
+        return best;
+    }
     // Automatic choice between the one-cell and the paired-cell kernel, from
     // B200 measurements (GLUPS, FP16 D3Q19, one-cell vs two-cell): pairs win
     // only on lattices without flags (BGK periodic 512^3: 64.3 vs 55.6).  With
@@ -241,9 +262,13 @@ struct cfdx_lbm {
     // 46.2 vs 45.6; D3Q27 Smagorinsky cavity 384^3 28.1 vs 34.7; gray channels
     // (D3Q19 128^3, D3Q27 256^3) 23.8 vs 37.5 and 12.8 vs 30.3 (the gray and
     // D3Q27 forms spill); periodic BGK 57.1 vs 63.7 for the flag-free paired
-    // kernel.  Automatic choice: where it wins.
-    static bool w2_default(int storage, int q, bool flags, bool gray) {
-        return storage == kStoreF16S && q == 19 && flags && !gray;
+    // kernel.  Below 2^20 cells its marches leave multiprocessors idle (us per
+    // step, pair / one-cell kernel: 32^3 LES cavity 7.4 / 4.9, 64^3 LES cavity 9.8 /
+    // 7.7, sphere pack 9.0 / 7.5, channel 7.1 / 7.4, 96^3 27.6 / 19.1, 27.0 / 20.0,
+    // 22.3 / 20.0; above: 300x60x60 channel 21.9 / 24.9, 128^3 channel 37.0 / 46.1,
+    // LES cavity 45.7 / 42.0).  Automatic choice: where it wins.
+    static bool w2_default(int storage, int q, bool flags, bool gray, std::size_t cells) {
+        return storage == kStoreF16S && q == 19 && flags && !gray && cells >= (std::size_t{1} << 20);
     }
     double les_k = 0.0;
     std::uint64_t h2d = 0, d2h = 0, syncs = 0;
@@ -317,7 +342,7 @@ struct cfdx_lbm {
         a.wall_mask = key.flags ? wall_mask : nullptr;
         a.near_list = key.flags ? near_list : nullptr;
         a.near_count = key.flags ? near_count : 0U;
-        a.planes = planes == 0U ? kDefaultPlanes : planes;
+        a.planes = planes == 0U ? auto_planes() : planes;
         a.ax_field = local_a;
         a.ay_field = local_a ? local_a + N : nullptr;
         a.az_field = local_a ? local_a + 2 * N : nullptr;
@@ -401,7 +426,7 @@ struct cfdx_lbm {
     void choose_variant() {
         key.narrow = offsets_fit();
         key.w2 = (variant == 3 || variant == 4 ||
-                  (variant == 0 && w2_default(key.storage, key.q, key.flags, key.gray))) &&
+                  (variant == 0 && w2_default(key.storage, key.q, key.flags, key.gray, N))) &&
                  w2_eligible();
         key.w2_pipe = variant != 4;
         key.paired = !key.w2 && (variant == 2 || (variant == 0 && paired_eligible() &&
@@ -519,12 +544,10 @@ void init_state(cfdx_lbm* h, const InitSpec& in) {
 
 void ensure_reduce(cfdx_lbm* h) {
     if (h->reduce_partials) return;
-    int sms = 0;
-    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->cfg.device), "device attribute");
     const long long rows = static_cast<long long>(h->cfg.ny * h->cfg.nz);
     const long long per_block = reduce_block(h->cfg.nx).y;
     h->reduce_blocks =
-        static_cast<int>(std::max(1LL, std::min<long long>(4LL * sms, (rows + per_block - 1) / per_block)));
+        static_cast<int>(std::max(1LL, std::min<long long>(4LL * h->sms, (rows + per_block - 1) / per_block)));
     // Pinned: the kernel's last block writes the sums straight to the host.
     if (!h->host_reduce) check_cuda(cudaMallocHost(&h->host_reduce, sizeof(double) * kReduceFields), "cudaMallocHost");
     // One row of partial sums per block, and one that holds the counter of finished blocks.
@@ -774,6 +797,7 @@ void build_handle(cfdx_lbm* h, const cfdx_lbm_config& c, const cfdx_lbm::Slab& s
                                         : double(reference_les_k()))
                                  : 0.0;
     default_scales(h);
+    check_cuda(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, c.device), "device attribute");
     check_cuda(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     check_cuda(cudaEventCreateWithFlags(&h->event, cudaEventDisableTiming), "cudaEventCreate");
     h->f_bytes = static_cast<std::size_t>(c.lattice) * h->N * static_cast<std::size_t>(storage_bytes(c.storage));
