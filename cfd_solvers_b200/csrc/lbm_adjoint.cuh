@@ -260,7 +260,8 @@ __global__ void __launch_bounds__(128, oop_min_blocks<L, S, GRAY>()) k_step_oop(
     dependent_begin();
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
-    const u32 z = blockIdx.z;
+    const u32 z = blockIdx.z, y0 = blockIdx.y * blockDim.y;
+    prefetch_rows<L, typename S::T>(f, z * f.ny + y0, min(blockDim.y, f.ny - y0));
     if (x >= f.nx || y >= f.ny) return;
     const u32 n = (z * f.ny + y) * f.nx + x;
     std::uint8_t flag = 0;
@@ -353,7 +354,9 @@ __global__ void __launch_bounds__(128, adjoint_min_blocks<L, S>()) k_adjoint_ste
     const LbmArgs& f = A.f;
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
-    const u32 z = blockIdx.z;
+    const u32 z = blockIdx.z, y0 = blockIdx.y * blockDim.y, rows = min(blockDim.y, f.ny - y0);
+    prefetch_rows<L, typename S::T>(f, z * f.ny + y0, rows);
+    prefetch_rows<L, typename LS::T>(A.l, z * f.ny + y0, rows);
     double g_tau = 0.0;
     if (x < f.nx && y < f.ny) {
         const u32 n = (z * f.ny + y) * f.nx + x;

@@ -90,6 +90,8 @@ struct LbmArgs {
     // separately).  Honoured by every step kernel (k_step, k_step_w2, k_step_h2,
     // k_step_x2); the other kernels cover the whole lattice.
     std::uint32_t z_first, z_end;
+    // Cells by which the step kernels' L2 prefetch runs ahead (0: none).
+    std::uint32_t ahead;
 };
 
 // Parameters of the adjoint kernels (lbm_adjoint.cuh).

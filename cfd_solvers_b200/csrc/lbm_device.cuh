@@ -484,6 +484,27 @@ __device__ __forceinline__ void scatter(const LbmArgs& a, u32 n, const Nbr& o, c
     scatter_pairs<L, S, NARROW, RAW>(a, n, o, fout, h);
 }
 
+// ----------------------------------------------------------------- prefetch
+// Asks L2 for the populations that lie a.ahead cells after the rows of this
+// block (`rows` of them from row index `row` on), one bulk request per
+// direction from the first block of the rows, so every row is asked for once
+// (whole rows: a request per 128 cells slowed D3Q27 down).  The kernels hold
+// their loads' latency with resident warps alone, and registers limit those.
+template <class L, class T> __device__ __forceinline__ void prefetch_rows(const LbmArgs& a, u32 row, u32 rows) {
+    const u32 d = threadIdx.y * blockDim.x + threadIdx.x;
+    if (a.ahead == 0U || blockIdx.x != 0U || d >= static_cast<u32>(L::Q)) return;
+    const unsigned long long m = static_cast<unsigned long long>(row) * a.nx + a.ahead;
+    const u32 cells = rows * a.nx;
+    if (m + cells + 16U > a.N) return; // whole 16-byte units inside the direction
+    // the request wants a 16-byte aligned address and size; the lattice itself may start at any
+    // element (the adjoint's frames lie one after the other)
+    const auto from = reinterpret_cast<unsigned long long>(static_cast<const T*>(a.base)) +
+                      (static_cast<unsigned long long>(d) * a.N + m) * sizeof(T);
+    const unsigned long long first = from & ~15ULL;
+    const u32 bytes = static_cast<u32>(((from + cells * sizeof(T) + 15ULL) & ~15ULL) - first);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(first), "r"(bytes));
+}
+
 // ------------------------------------------------------------------ helpers
 // Reciprocals.  rcp: the hardware approximation (within 1 ulp), for relaxation
 // rates, which enter a cell's mass and momentum alike; flushing, because
@@ -1098,6 +1119,10 @@ __global__ void __launch_bounds__(128, step_min_blocks<L, S, GRAY>()) k_step(con
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z0 = a.z_first + blockIdx.z * CPT;
+    if constexpr (!IsAudit<S>::value && sizeof(typename S::T) >= 4) {
+        const u32 y0 = blockIdx.y * blockDim.y;
+        prefetch_rows<L, typename S::T>(a, z0 * a.ny + y0, min(blockDim.y, a.ny - y0));
+    }
     if (x >= a.nx || y >= a.ny) return;
     R fin[CPT][L::Q];
     std::uint8_t flag[CPT];

@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(128, LES ? CFDX_H2_MIN_BLOCKS_LES : CFDX_H2_MI
     H2Ctx c;
     c.x0 = 2U * (blockIdx.x * blockDim.x + threadIdx.x);
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
-    const u32 z = a.z_first + blockIdx.z;
+    const u32 z = a.z_first + blockIdx.z, yb = blockIdx.y * blockDim.y;
+    prefetch_rows<L, __half>(a, z * a.ny + yb, min(blockDim.y, a.ny - yb));
     if (c.x0 >= a.nx || y >= a.ny) return;
     c.row = (z * a.ny + y) * a.nx;
     c.n0 = c.row + c.x0;
