@@ -914,7 +914,11 @@ CFDX_API int cfdx_lbm_init_fields(cfdx_lbm* h, const float* fields, int where) {
         require(fields != nullptr, "null fields");
         InitSpec s{};
         s.kind = 2;
-        if (where == CFDX_DEVICE && local_device_memory(fields, h->cfg.device, sizeof(float))) {
+        // Device fields are read in place, unless they lie in the lattice they initialise.
+        const auto* first = reinterpret_cast<const char*>(fields);
+        const auto* lattice = static_cast<const char*>(h->f);
+        const bool apart = first >= lattice + h->f_bytes || first + 4U * h->N * sizeof(float) <= lattice;
+        if (where == CFDX_DEVICE && apart && local_device_memory(fields, h->cfg.device, sizeof(float))) {
             s.fields = fields;
             init_state(h, s);
             h->sync(); // the caller may reuse its buffer on return
