@@ -883,22 +883,28 @@ template <class Coef, int E> constexpr bool v_any() {
         if (Coef::at(p) != 0) return true;
     return false;
 }
-// Sum over the weight classes in storage units of class 2: sum_k (s_2 / s_k)
-// sum_k-class(v), with r1 = s_2 / s_1 and r3 = s_2 / s_3 (exact for the default
-// power-of-two scales).  One multiply-add per class beyond the second; classes
-// without a term (c_a c_b = 0 for the axis pairs when a != b) cost nothing.
+// init + sum_k sum_k-class(v) / s_k over the weight classes 1..K in that order, as a
+// multiply-add chain; classes without a term (c_a c_b = 0 for the axis pairs when
+// a != b) cost nothing.  The order is part of the results: a moment that rounds
+// otherwise turns into another stored half now and then, and a restarted FP16 run
+// leaves the trajectory it had.  Summing in units of class 2, one multiply-add less
+// per moment, moved 256^3 Smagorinsky cavities by 2.9e-4 (D3Q19) and 1.1e-4 (D3Q27)
+// within a case's steps and gave little (B200, us per step, this form / that one:
+// D3Q27 256^3 510 / 500, D3Q19 256^3 339.2 / 338.8, 512x256x256 sphere pack 699 / 707).
 template <class Coef1, class Coef2, class Coef3, class L, class V>
-__device__ __forceinline__ V class_blend(const V* v, float r1, float r3) {
-    V r = v_csum<Coef2, 0, L::PAIRS>(v);
-    if constexpr (v_any<Coef1, L::PAIRS>()) r = v_fma(v_csum<Coef1, 0, L::PAIRS>(v), v_splat<V>(r1), r);
-    if constexpr (L::Q == 27) r = v_fma(v_csum<Coef3, 0, L::PAIRS>(v), v_splat<V>(r3), r);
+__device__ __forceinline__ V class_chain(const V* v, const float* inv, V init) {
+    V r = init;
+    if constexpr (v_any<Coef1, L::PAIRS>()) r = v_fma(v_csum<Coef1, 0, L::PAIRS>(v), v_splat<V>(inv[1]), r);
+    r = v_fma(v_csum<Coef2, 0, L::PAIRS>(v), v_splat<V>(inv[2]), r);
+    if constexpr (L::Q == 27) r = v_fma(v_csum<Coef3, 0, L::PAIRS>(v), v_splat<V>(inv[3]), r);
     return r;
 }
-template <class L, int A, class V> __device__ __forceinline__ V blend1(const V* v, float r1, float r3) {
-    return class_blend<CoefFirst<L, 1, A>, CoefFirst<L, 2, A>, CoefFirst<L, 3, A>, L>(v, r1, r3);
+template <class L, int A, class V> __device__ __forceinline__ V scaled_moment(const V* v, const float* inv, V init) {
+    return class_chain<CoefFirst<L, 1, A>, CoefFirst<L, 2, A>, CoefFirst<L, 3, A>, L>(v, inv, init);
 }
-template <class L, int A, int B, class V> __device__ __forceinline__ V blend2(const V* v, float r1, float r3) {
-    return class_blend<CoefSecond<L, 1, A, B>, CoefSecond<L, 2, A, B>, CoefSecond<L, 3, A, B>, L>(v, r1, r3);
+template <class L, int A, int B, class V>
+__device__ __forceinline__ V scaled_moment2(const V* v, const float* inv, V init) {
+    return class_chain<CoefSecond<L, 1, A, B>, CoefSecond<L, 2, A, B>, CoefSecond<L, 3, A, B>, L>(v, inv, init);
 }
 
 // sqrt for the Smagorinsky rate: hardware reciprocal square root (2 ulp);
@@ -927,14 +933,11 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
         inv[k] = a.inv_scale[class_rep(k)];
         scl[k] = a.scale[class_rep(k)];
     }
-    const V inv2 = v_splat<V>(inv[2]);
-    const float r1 = __fmul_rn(inv[1], scl[2]), r3 = L::Q == 27 ? __fmul_rn(inv[K], scl[2]) : 0.0F;
-    const V rho = v_add(v_fma(blend1<L, 0>(sh, r1, r3), inv2, v_mul(h[0], v_splat<V>(inv[0]))), one);
+    const V rho = v_add(scaled_moment<L, 0>(sh, inv, v_mul(h[0], v_splat<V>(inv[0]))), one);
     const V zero = v_splat<V>(-0.0F); // x + (-0) == x for every x
     const V irho = v_map(rho, [](float r, int) { return r > 0.0F ? rcp_unbiased(r) : 0.0F; });
-    const V irho2 = v_mul(irho, inv2); // 1 / (rho s_2)
-    V ux = v_mul(blend1<L, 1>(dh, r1, r3), irho2), uy = v_mul(blend1<L, 2>(dh, r1, r3), irho2),
-      uz = v_mul(blend1<L, 3>(dh, r1, r3), irho2);
+    V ux = v_mul(scaled_moment<L, 1>(dh, inv, zero), irho), uy = v_mul(scaled_moment<L, 2>(dh, inv, zero), irho),
+      uz = v_mul(scaled_moment<L, 3>(dh, inv, zero), irho);
     V ax = zero, ay = zero, az = zero;
     if constexpr (FORCE) {
         ax = v_map(ax, [&](float, int k) { float x, y, z; cell_acceleration<float>(a, n + k, x, y, z); return x; });
@@ -948,17 +951,17 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
     V omega, omega_m;
     if constexpr (LES) {
         const V third = v_splat<V>(1.0F / 3.0F);
-        const V sxx = v_fma(blend2<L, 1, 1>(sh, r1, r3), inv2, third);
-        const V syy = v_fma(blend2<L, 2, 2>(sh, r1, r3), inv2, third);
-        const V szz = v_fma(blend2<L, 3, 3>(sh, r1, r3), inv2, third);
+        const V sxx = scaled_moment2<L, 1, 1>(sh, inv, third);
+        const V syy = scaled_moment2<L, 2, 2>(sh, inv, third);
+        const V szz = scaled_moment2<L, 3, 3>(sh, inv, third);
         const V nrho = v_mul(rho, v_splat<V>(-1.0F));
         const V pxx = v_fma(nrho, v_fma(ux, ux, third), sxx);
         const V pyy = v_fma(nrho, v_fma(uy, uy, third), syy);
         const V pzz = v_fma(nrho, v_fma(uz, uz, third), szz);
         const V nrux = v_mul(nrho, ux), nruy = v_mul(nrho, uy);
-        const V pxy = v_fma(blend2<L, 1, 2>(sh, r1, r3), inv2, v_mul(nrux, uy));
-        const V pxz = v_fma(blend2<L, 1, 3>(sh, r1, r3), inv2, v_mul(nrux, uz));
-        const V pyz = v_fma(blend2<L, 2, 3>(sh, r1, r3), inv2, v_mul(nruy, uz));
+        const V pxy = v_fma(nrux, uy, scaled_moment2<L, 1, 2>(sh, inv, zero));
+        const V pxz = v_fma(nrux, uz, scaled_moment2<L, 1, 3>(sh, inv, zero));
+        const V pyz = v_fma(nruy, uz, scaled_moment2<L, 2, 3>(sh, inv, zero));
         V off = v_mul(pxy, pxy);
         off = v_fma(pxz, pxz, off);
         off = v_fma(pyz, pyz, off);
