@@ -438,13 +438,16 @@ __device__ __forceinline__ u32 cell_index(long long i, u32 extent) {
 }
 
 // The values at x0 and x0 + 1 of a row.  PAIRS: rows start 8-byte aligned (even
-// nx, aligned fields), so an even x0 below the last takes one 8-byte access.
+// nx, aligned fields), so an even x0 (`joint`; its right neighbour never wraps)
+// takes one 8-byte access; an odd one loads its pair and the one after it.
 template <bool PAIRS> __device__ __forceinline__ float2 row_pair(const float* f, u32 n0, u32 n1, bool joint) {
-    if (PAIRS && joint) return *reinterpret_cast<const float2*>(f + n0);
-    return make_float2(f[n0], f[n1]);
+    if constexpr (!PAIRS) return make_float2(f[n0], f[n1]);
+    float2 q = *reinterpret_cast<const float2*>(f + (n0 & ~1U));
+    if (!joint) q = make_float2(q.y, f[n1]);
+    return q;
 }
-template <bool PAIRS> __device__ __forceinline__ void add_pair(float* f, u32 n0, u32 n1, bool joint, float a, float b) {
-    if (PAIRS && joint) {
+__device__ __forceinline__ void add_pair(float* f, u32 n0, u32 n1, bool joint, float a, float b) {
+    if (joint) {
         atomicAdd(reinterpret_cast<float2*>(f + n0), make_float2(a, b));
     } else {
         atomicAdd(f + n0, a);
@@ -452,18 +455,52 @@ template <bool PAIRS> __device__ __forceinline__ void add_pair(float* f, u32 n0,
     }
 }
 
-__device__ __forceinline__ float warp_total(float v) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffU, v, s);
+// Sums over the lanes of a warp that share a cell, for all groups of lanes at once:
+// in each round every remaining lane of even rank in its group takes the value
+// of the next one, so the group's first lane holds its sum after log2(largest
+// group) rounds.  The rounds are worked out once per particle and used for
+// every value: `from` holds 6 bits per round (5 of the lane to take from, and
+// whether to take), `rounds` is the same in every lane.
+struct CellGroup {
+    unsigned lanes; // the lanes that take part
+    u32 from;
+    int rounds;
+    bool first;     // of its group
+};
+__device__ __forceinline__ CellGroup cell_group(u32 cell) {
+    CellGroup g{__activemask(), 0U, 0, false};
+    const unsigned lane = threadIdx.x & 31U;
+    const unsigned peers = __match_any_sync(g.lanes, cell);
+    unsigned rank = __popc(peers & ((1U << lane) - 1U));
+    g.first = rank == 0U;
+    for (unsigned later = peers & (0xfffffffeU << lane); __any_sync(g.lanes, later != 0U); ++g.rounds) {
+        const unsigned take = later ? 32U + (__ffs(later) - 1U) : lane;
+        g.from |= take << (6 * g.rounds);
+        later &= __ballot_sync(g.lanes, (rank & 1U) == 0U); // the others have been taken
+        rank >>= 1;
+    }
+    return g;
+}
+__device__ __forceinline__ float group_sum(const CellGroup& g, float v) {
+    for (int k = 0; k < g.rounds; ++k) {
+        const u32 take = g.from >> (6 * k);
+        const float t = __shfl_sync(g.lanes, v, static_cast<int>(take & 31U));
+        if (take & 32U) v = __fadd_rn(v, t);
+    }
     return v;
 }
 
 // Bound by the latency and the sectors of its scattered accesses (24 loads and
-// 24 additions per particle, each lane in a sector of its own).  2^18 particles
-// at random in 192^3 cells: 90.5 us with joint accesses and 32-bit indices, 100.4
-// with a scalar access per corner and 64-bit remainders (B200); more resident
-// blocks (10, 12 per SM) change nothing.  All 2^18 in one cell: 23.5 us with the
-// warp's sum added once, 1164 with an addition per particle.
+// 24 additions per particle, each lane in a sector of its own), and by the queue
+// at one address where particles gather.  2^18 particles in 192^3 cells, two-way,
+// us per call (B200; in brackets one scalar access per corner and particle): at
+// random 102 (112), in one plane 50 (64), at random in a ball of radius 4 86 (110),
+// in 512 cells 42 (49), 64 cells 62 (84), 8 cells 67 (226), one cell 26 (1168), one cell with
+// a stray in every warp 28 (1124).  191 x 192 x 192, without joint accesses: 109 (112),
+// 60 (62), 111 (117), 52 (50), 72 (83), 71 (231), 49 (1322), 51 (1270).  Summing only
+// where three or five lanes share a cell is slower (64 cells 65 and 76), and so is
+// a sum only for warps in one cell (8 cells 256).  More resident blocks (10, 12
+// per SM) change nothing.
 template <bool PAIRS>
 __global__ void __launch_bounds__(128, 8) k_particles(float* st, u32 count, ThermalGrid t, const float* ux,
                                                        const float* uy, const float* uz, float* ax, float* ay,
@@ -478,7 +515,7 @@ __global__ void __launch_bounds__(128, 8) k_particles(float* st, u32 count, Ther
     const float tx = __fsub_rn(px, float(x0)), ty = __fsub_rn(py, float(y0)), tz = __fsub_rn(pz, float(z0));
     const u32 xi = cell_index(x0, t.nx), yi = cell_index(y0, t.ny), zi = cell_index(z0, t.nz);
     const u32 xn = shp(xi, t.nx), ys[2] = {yi, shp(yi, t.ny)}, zs[2] = {zi, shp(zi, t.nz)};
-    const bool joint = (xi & 1U) == 0U && xn == xi + 1U;
+    const bool joint = (xi & 1U) == 0U;
     const float wx[2] = {__fsub_rn(1.0F, tx), tx}, wy[2] = {__fsub_rn(1.0F, ty), ty}, wz[2] = {__fsub_rn(1.0F, tz), tz};
     float2 u[4], v[4], w[4];
 #pragma unroll
@@ -503,13 +540,9 @@ __global__ void __launch_bounds__(128, 8) k_particles(float* st, u32 count, Ther
     const float dragy = __fdiv_rn(__fmul_rn(mass, __fsub_rn(fv, vy)), response);
     const float dragz = __fdiv_rn(__fmul_rn(mass, __fsub_rn(fw, vz)), response);
     if (two_way) {
-        // particles that settled into one cell (or lost their position) would all add to the same
-        // eight cells: a warp that shares its cell adds its sum
-        const unsigned lanes = __activemask();
-        int one_cell = 0;
-        __match_all_sync(lanes, (zi * t.ny + yi) * t.nx + xi, &one_cell);
-        const bool shared = one_cell != 0 && lanes == 0xffffffffU;
-        const bool adds = !shared || (threadIdx.x & 31U) == 0U;
+        // particles that gather in few cells (settled, or without a finite position) would queue at
+        // the same additions: the lanes of a warp that share a cell add their sum once
+        const CellGroup group = cell_group((zi * t.ny + yi) * t.nx + xi);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const u32 row = (zs[r >> 1] * t.ny + ys[r & 1]) * t.nx;
@@ -517,14 +550,25 @@ __global__ void __launch_bounds__(128, 8) k_particles(float* st, u32 count, Ther
             const float b = __fmul_rn(__fmul_rn(wx[1], wy[r & 1]), wz[r >> 1]);
             const float drag[3] = {-dragx, -dragy, -dragz};
             float* const field[3] = {ax, ay, az};
+            if constexpr (PAIRS) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                float lo = __fmul_rn(drag[k], a), hi = __fmul_rn(drag[k], b);
-                if (shared) {
-                    lo = warp_total(lo);
-                    hi = warp_total(hi);
+                for (int k = 0; k < 3; ++k) {
+                    float lo = __fmul_rn(drag[k], a), hi = __fmul_rn(drag[k], b);
+                    if (group.rounds > 0) {
+                        lo = group_sum(group, lo);
+                        hi = group_sum(group, hi);
+                    }
+                    if (group.first) add_pair(field[k], row + xi, row + xn, joint, lo, hi);
                 }
-                if (adds) add_pair<PAIRS>(field[k], row + xi, row + xn, joint, lo, hi);
+            } else { // corner by corner, the three fields in turn
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        float v = __fmul_rn(drag[k], c ? b : a);
+                        if (group.rounds > 0) v = group_sum(group, v);
+                        if (group.first) atomicAdd(field[k] + row + (c ? xn : xi), v);
+                    }
             }
         }
     }
