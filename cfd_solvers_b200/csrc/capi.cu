@@ -53,8 +53,15 @@ void check_cuda(cudaError_t e, const char* what) {
     fail(CFDX_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// Allocation wrapper with the test hook of cfdx_debug_fail_allocations().
-void* device_alloc(std::size_t bytes, const char* what) {
+// Device memory from `allocate` (which sets *p), with the test hooks of
+// cfdx_debug_fail_allocations() and cfdx_debug_retry_allocations().  Out of
+// memory: the scratch pool may hold idle memory from earlier voxelizer,
+// Q-criterion or flag calls; it goes back to the driver, and the allocation is
+// tried once more.  No synchronisation: the trim releases what the pool holds idle
+// now, and pool memory whose stream-ordered free has not run yet stays mapped
+// (waiting for every stream of the device would stall other handles and other
+// libraries).
+template <class F> void* allocate_or_retry(const char* what, F&& allocate) {
     if (g_fail_allocations.load() > 0) {
         g_fail_allocations.fetch_sub(1);
         fail(CFDX_ERR_OOM, std::string(what) + ": injected allocation failure (cudaErrorMemoryAllocation)");
@@ -65,22 +72,20 @@ void* device_alloc(std::size_t bytes, const char* what) {
         g_retry_allocations.fetch_sub(1);
         e = cudaErrorMemoryAllocation; // test hook: the first attempt reports out-of-memory
     } else {
-        e = cudaMalloc(&p, bytes);
+        e = allocate(&p);
     }
     if (e == cudaErrorMemoryAllocation) {
-        // The scratch pool may hold idle memory from earlier voxelizer / Q-criterion
-        // calls: return it to the driver and try once more.  No synchronisation:
-        // the trim releases what the pool holds idle now, and pool memory whose
-        // stream-ordered free has not run yet stays mapped (waiting for every
-        // stream of the device would stall other handles and other libraries).
         cudaGetLastError();
         ++g_allocation_retries;
         int device = 0;
-        if (cudaGetDevice(&device) == cudaSuccess && scratch_release(device) == cudaSuccess)
-            e = cudaMalloc(&p, bytes);
+        if (cudaGetDevice(&device) == cudaSuccess && scratch_release(device) == cudaSuccess) e = allocate(&p);
     }
     check_cuda(e, what);
     return p;
+}
+
+void* device_alloc(std::size_t bytes, const char* what) {
+    return allocate_or_retry(what, [&](void** p) { return cudaMalloc(p, bytes); });
 }
 
 void device_free(void* p) {
@@ -89,16 +94,12 @@ void device_free(void* p) {
 
 // Device scratch of one call from the per-device pool (scratch_pool.cu), in
 // stream order: no cudaMalloc mapping and no device-wide cudaFree
-// synchronisation per call.  Honours the allocation-failure test hook.
+// synchronisation per call.
 struct StageBuffer {
     void* p = nullptr;
     cudaStream_t s;
     StageBuffer(cudaStream_t stream, std::size_t bytes, const char* what) : s(stream) {
-        if (g_fail_allocations.load() > 0) {
-            g_fail_allocations.fetch_sub(1);
-            fail(CFDX_ERR_OOM, std::string(what) + ": injected allocation failure (cudaErrorMemoryAllocation)");
-        }
-        check_cuda(scratch_alloc(&p, bytes, s), what);
+        p = allocate_or_retry(what, [&](void** q) { return scratch_alloc(q, bytes, s); });
     }
     StageBuffer(const StageBuffer&) = delete;
     StageBuffer& operator=(const StageBuffer&) = delete;

@@ -1,5 +1,5 @@
 // Per-device, stream-ordered memory pool for the temporary buffers of single
-// calls (voxelizer scratch, Q-criterion staging): scratch_pool.cu.
+// calls (voxelizer scratch, Q-criterion and flag staging): scratch_pool.cu.
 #pragma once
 
 #include <cstddef>

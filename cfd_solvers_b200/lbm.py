@@ -552,8 +552,8 @@ class EsotericPullCudaSolver:
 
 def release_scratch(device: int = 0, library=None):
     """Return the unused memory of the library's per-device scratch pool to the driver
-    (cfdx_release_scratch).  The voxelizer and the Q-criterion take their temporary buffers from
-    that pool, which keeps up to 8 GiB mapped between calls."""
+    (cfdx_release_scratch).  The voxelizer, the Q-criterion and set_flags take their temporary
+    buffers from that pool, which keeps up to 8 GiB mapped between calls."""
     lib = library or B.load()
     lib.call("cfdx_release_scratch", int(device))
 

@@ -586,10 +586,13 @@ CFDX_API int cfdx_diagnostics_q_criterion(cfdx_diagnostics* diagnostics, const f
 CFDX_API int cfdx_diagnostics_info(cfdx_diagnostics* diagnostics, size_t* resident_bytes);
 
 /* Temporary buffers of single calls (cfdx_voxelize / cfdx_lbm_set_flags_surface
- * scratch, cfdx_q_criterion / cfdx_lbm_q_criterion staging) come from a
- * stream-ordered memory pool the library keeps per device, which keeps up to
- * 8 GiB mapped between calls so that repeated calls do not map memory anew or
- * synchronise the device in cudaFree.  This returns the pool's unused memory on
+ * scratch, cfdx_q_criterion / cfdx_lbm_q_criterion staging, and the staging of
+ * cfdx_lbm_set_flags: one byte per cell for host flags, 256 bytes for device
+ * flags) come from a stream-ordered memory pool the library keeps per device, which
+ * keeps up to 8 GiB mapped between calls so that repeated calls do not map memory
+ * anew or synchronise the device in cudaFree.  An allocation of the library that
+ * runs out of memory hands the pool's unused memory back and tries again; other
+ * libraries' allocations cannot.  This returns the pool's unused memory on
  * `device` to the driver (after synchronising the device). */
 CFDX_API int cfdx_release_scratch(int device);
 

@@ -156,3 +156,38 @@ def test_fields_inside_the_lattice_are_staged(engine):
             s.step(2)
             out.append(s.logical_populations())
     assert np.array_equal(out[0], out[1])
+
+
+def test_flag_staging_retries_when_memory_is_short(engine):
+    """Host flags and voxelized bodies are staged from the scratch pool: a first attempt that runs out of
+    memory returns the pool's idle memory and tries again, as every other allocation does."""
+    cs = engine
+    lib = cs.load()
+    nx, ny, nz = 17, 6, 5
+    flags = random_flags((nz, ny, nx), 9)
+    triangles = np.array([[[0.1, 0.1, 0.1], [0.9, 0.1, 0.1], [0.1, 0.9, 0.1]]])
+
+    def retries():
+        count = ctypes.c_ulonglong(0)
+        lib.raw.cfdx_debug_retry_allocations(-1, ctypes.byref(count))
+        return count.value
+
+    with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=nx, ny=ny, nz=nz)) as s:
+        s.set_flags(np.zeros(flags.size, np.uint8))  # holds its flag and wall-link fields from here on
+        want = None
+        for hook in (0, 1):
+            before = retries()
+            lib.raw.cfdx_debug_retry_allocations(hook, None)
+            try:
+                s.set_flags(flags)
+                s.initialize_uniform(1.0, 0.02, 0.0, 0.0)
+                s.step(2)
+                got = s.logical_populations()
+                assert retries() == before + hook
+                lib.raw.cfdx_debug_retry_allocations(hook, None)
+                s.set_solid_surface(triangles)
+                assert retries() == before + 2 * hook
+            finally:
+                lib.raw.cfdx_debug_retry_allocations(0, None)
+            want = got if want is None else want
+            assert np.array_equal(got, want)
