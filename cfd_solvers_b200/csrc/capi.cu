@@ -49,6 +49,9 @@ struct CfdxError : std::runtime_error {
 
 void check_cuda(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return;
+    // This report takes the error: the runtime keeps it as its last one as well, where the next
+    // launch's check (of this library or another) would find it.
+    cudaGetLastError();
     if (e == cudaErrorMemoryAllocation) fail(CFDX_ERR_OOM, std::string(what) + ": " + cudaGetErrorString(e));
     fail(CFDX_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -191,3 +191,15 @@ def test_flag_staging_retries_when_memory_is_short(engine):
                 lib.raw.cfdx_debug_retry_allocations(0, None)
             want = got if want is None else want
             assert np.array_equal(got, want)
+
+
+def test_an_allocation_that_fails_leaves_no_error_behind(engine):
+    """A lattice larger than the device is refused; the launches after it do not report that error again."""
+    cs = engine
+    with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=18, ny=7, nz=5)) as s:
+        with pytest.raises(MemoryError):
+            cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=1500, ny=1500, nz=1500, lattice="d3q27", storage="fp64"))
+        s.set_flags(random_flags((5, 7, 18), 3))
+        s.initialize_uniform()
+        s.step(2)
+        assert s.reduce()["nonfinite"] == 0
