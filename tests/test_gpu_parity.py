@@ -264,7 +264,8 @@ def test_fp16_storage_matches_fp16_oracle(engine, oracle_mod, q, wide):
         assert fields_err(s.compute_macroscopic(), L.macroscopic()) < 5e-5
 
 
-FP16_WALL_CASES = [("sphere", (96, 40, 36)), ("sphere", (256, 24, 20)), ("cavity", (96, 96, 96))]
+FP16_WALL_CASES = [("sphere", (96, 40, 36)), ("sphere", (256, 24, 20)), ("cavity", (96, 96, 96)),
+                   ("sphere", (256, 66, 64)), ("cavity", (104, 102, 100))]
 
 
 @pytest.mark.parametrize("case, shape", FP16_WALL_CASES, ids=[f"{c}-{a}x{b}x{d}" for c, (a, b, d) in FP16_WALL_CASES])
@@ -273,9 +274,10 @@ def test_fp16_walled_lattices_match_fp16_oracle(engine, oracle_mod, case, shape,
     """The shapes of the precision configuration (a D3Q19 TRT channel, periodic in x with no-slip
     y/z walls, a seeded sphere pack, a body force) and of the plain method at scale (a lid-driven
     cavity, TRT + Smagorinsky Cs 0.1, tau 0.51, lid (0.1, 0, 0)) in FP16 shifted storage, on lattices
-    the oracle runs in seconds (nearest rounding, the oracle's codec).  With flags and an even nx the
-    automatic step is the wall-aware pair kernel, so its near-wall pairs are checked against the
-    oracle directly: wall cells beside fluid cells in one pair (every x-wall of the cavity), fluid
+    the oracle runs in seconds (nearest rounding, the oracle's codec).  The automatic
+    step is the one-cell kernel on the first three lattices and, from 2^20 cells on, the wall-aware pair
+    kernel on the last two; forced, it runs on all five. So its near-wall pairs are checked against
+    the oracle directly: wall cells beside fluid cells in one pair (every x-wall of the cavity), fluid
     pairs that disagree on a wall link (sphere surfaces), shifted words that wrap around x beside a
     sphere, and the rows next to the moving lid.  9 and 10 steps."""
     from cfd_solvers_b200.cases import sphere_pack

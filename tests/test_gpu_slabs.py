@@ -55,6 +55,8 @@ def setup(cs, q=19, shape=(12, 10, 13), storage="fp32", coll="trt", les=False, w
 
 def prepare(s, inputs, local=None):
     pick = local or (lambda a, k=1: a)
+    if "planes" in inputs:
+        s.set_step_planes(inputs["planes"])
     if "flags" in inputs:
         s.set_flags(pick(inputs["flags"]))
         s.set_wall_velocity(3, 0.03, 0.0, -0.01)
@@ -172,6 +174,16 @@ def test_two_phase_step_matches_whole_lattice(engine, mode, q, storage, variant,
     cfg, inputs = setup(engine, q=q, shape=(16, 9, 13), storage=storage, les=True, gray=variant != 3,
                         local_force=True)
     check(engine, cfg, inputs, ranks, steps=5, mode=mode, variant=variant)
+
+
+@pytest.mark.parametrize("mode", ["direct", "phases"])
+@pytest.mark.parametrize("planes", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("ranks", [1, 2, 5])
+def test_pair_kernel_marches_in_slabs(engine, mode, planes, ranks):
+    """The wall-aware pair kernel at given planes per thread: slabs of 17, 9 and 8, 4 and 3 planes,
+    whose interiors end its marches at every depth."""
+    cfg, inputs = setup(engine, q=19, shape=(34, 9, 17), storage="fp16s", les=True, local_force=True)
+    check(engine, cfg, dict(inputs, planes=planes), ranks, steps=5, mode=mode, variant=3)
 
 
 def test_two_phase_step_order_is_enforced(engine):

@@ -93,15 +93,17 @@ def test_cached_graph_follows_changes(engine):
 
 
 @pytest.mark.parametrize("q, storage, variant", [(19, "fp32", 0), (19, "fp32", 2), (27, "fp32", 0), (19, "fp64", 0),
-                                                 (19, "fp16s", 0), (19, "fp16s", 1), (19, "fp16s", 2), (27, "fp16s", 0)])
-def test_overlapping_launches_equal_separate_ones(engine, q, storage, variant):
-    """Each lattice kernel may be scheduled while the one before it drains (programmatic dependent
-    launch): steps, reductions, field reads and setters queued back to back equal the same calls
+                                                 (19, "fp16s", 0), (19, "fp16s", 1), (19, "fp16s", 2), (27, "fp16s", 0),
+                                                 (19, "fp16s", 3), (19, "fp16s", 4), (27, "fp16s", 3)])
+@pytest.mark.parametrize("kind", ["gray", "cavity", "periodic"])
+def test_overlapping_launches_equal_separate_ones(engine, q, storage, variant, kind):
+    """Each lattice kernel, in its gray, walled and open form, may be scheduled while the one before
+    it drains (programmatic dependent launch): steps, reductions, field reads and setters queued back to back equal the same calls
     with the stream drained after each, bit for bit."""
     cs = engine
     out = []
     for drain in (False, True):
-        with solver(cs, q, storage, "gray", variant) as s:
+        with solver(cs, q, storage, kind, variant) as s:
             seen = []
             for k in range(12):
                 s.step(1 + 9 * (k % 3))

@@ -88,6 +88,36 @@ def test_wall_aware_pairs_match_single_bitwise(engine, q, storage, shape, flags_
     assert a_red["mass"] == b_red["mass"]
 
 
+# Marches of four planes and more, the lengths that large lattices take: only from the fourth plane
+# on does the pipelined form store all four slots of its flag ring and fetch wall-link masks
+# three planes ahead over the stage it has just read.  Whole chunks and short last ones.
+LONG_SHAPES = [(18, 7, 17), (130, 6, 8), (256, 5, 21)]
+
+
+@pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("storage", ["fp16s", "fp16s:nearest"])
+@pytest.mark.parametrize("shape", LONG_SHAPES, ids=[f"{a}x{b}x{c}" for a, b, c in LONG_SHAPES])
+@pytest.mark.parametrize("flags_kind, gray", [(None, False), ("random", False), ("random", True), ("cavity", False)])
+@pytest.mark.parametrize("variant, planes", [(3, 4), (3, 5), (3, 8), (3, 21), (4, 4)])
+def test_wall_aware_pairs_in_long_marches(engine, q, storage, shape, flags_kind, gray, variant, planes):
+    a_log, a_red = run(engine, 1, q, shape, storage, flags_kind, gray, 5)
+    b_log, b_red = run(engine, variant, q, shape, storage, flags_kind, gray, 5, planes=planes)
+    assert np.array_equal(a_log.view(np.uint32), b_log.view(np.uint32))
+    assert a_red["mass"] == b_red["mass"]
+
+
+# Above 2^20 cells a walled D3Q19 FP16 lattice takes the pair kernel, with the planes per thread that
+# the rule picks for its size (four on the last shape).
+@pytest.mark.parametrize("shape", [(104, 102, 100), (300, 60, 60), (256, 160, 128)], ids=str)
+@pytest.mark.parametrize("flags_kind", ["random", "cavity"])
+def test_automatic_choice_above_the_border_matches_single_bitwise(engine, shape, flags_kind):
+    assert np.prod(shape) >= 1 << 20
+    a_log, a_red = run(engine, 1, 19, shape, "fp16s", flags_kind, False, 3)
+    b_log, b_red = run(engine, 0, 19, shape, "fp16s", flags_kind, False, 3)
+    assert np.array_equal(a_log.view(np.uint32), b_log.view(np.uint32))
+    assert a_red["mass"] == b_red["mass"]
+
+
 def test_wall_aware_pairs_need_fp16_and_even_nx(engine):
     cs = engine
     with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=16, ny=4, nz=4)) as s:
