@@ -232,7 +232,7 @@ struct cfdx_lbm {
     // longer tail: about one block's march on top of its share of the work, at
     // five resident blocks per SM.  B200, us per step at 4 / 3 / 2 / 1 planes:
     // LES cavities 512^3 2395 / 2404 / 2437 / 2758, 256^3 329 / 330 / 325 / -, 128^3
-    // 48.9 / 46.7 / 44.4 / 44.2, 64^3 24.3 / 16.2 / 13.5 / 9.8; sphere packs
+    // 48.9 / 46.7 / 44.4 / 44.2 (short bursts; 46 at the rule's 2 under load), 64^3 24.3 / 16.2 / 13.5 / 9.8; sphere packs
     // 512x256x256 686 / 695 / 716 / -, 100x90x80 25.4 / 24.6 / 23.1 / 22.4.
     std::uint32_t auto_planes() const {
         const std::size_t across = (cfg.nx / 2U + 31U) / 32U * ((cfg.ny + 3U) / 4U);
@@ -259,18 +259,22 @@ struct cfdx_lbm {
     static bool paired_default(int storage, int q, bool flags) {
         return storage == kStoreF16S && q == 19 && !flags;
     }
-    // The wall-aware z-marching pair kernel (k_step_w2, cp.async pipeline, 4
-    // planes per thread, wall links resolved three planes ahead) against the
-    // one-cell kernel, B200, FP16, GLUPS: D3Q19 TRT + Smagorinsky cavity 512^3
-    // 52.2 vs 47.8; without Smagorinsky 53.3 vs 51.4; 512x256x256 sphere pack
-    // 46.2 vs 45.6; D3Q27 Smagorinsky cavity 384^3 28.1 vs 34.7; gray channels
-    // (D3Q19 128^3, D3Q27 256^3) 23.8 vs 37.5 and 12.8 vs 30.3 (the gray and
-    // D3Q27 forms spill); periodic BGK 57.1 vs 63.7 for the flag-free paired
-    // kernel.  Below 2^20 cells its marches leave multiprocessors idle (us per
-    // step, pair / one-cell kernel: 32^3 LES cavity 7.4 / 4.9, 64^3 LES cavity 9.8 /
-    // 7.7, sphere pack 9.0 / 7.5, channel 7.1 / 7.4, 96^3 27.6 / 19.1, 27.0 / 20.0,
-    // 22.3 / 20.0; above: 300x60x60 channel 21.9 / 24.9, 128^3 channel 37.0 / 46.1,
-    // LES cavity 45.7 / 42.0).  Automatic choice: where it wins.
+    // The wall-aware z-marching pair kernel (k_step_w2, cp.async pipeline, planes
+    // per thread by auto_planes, wall links resolved three planes ahead) against the
+    // one-cell kernel.  It loses in its gray and D3Q27 forms, which spill (GLUPS:
+    // gray channels D3Q19 128^3 and D3Q27 256^3 23.8 vs 37.5 and 12.8 vs 30.3, D3Q27
+    // Smagorinsky cavity 384^3 28.1 vs 34.7), and to the flag-free paired kernel on
+    // periodic BGK (57.1 vs 63.7).  D3Q19 with walls, us per step on B200, pair /
+    // one-cell:
+    //   no Smagorinsky: channels 32^3 4.8 / 3.5, 64^3 7.0 / 7.6, 96^3 22.2 / 20.4,
+    //     300x60x60 21.8 / 25.4, 128^3 36.9 / 46.8, 160^3 88.6 / 98.0, 256x192x192 178 / 222;
+    //     sphere packs 96^3 26.9 / 20.4, 256x128x128 93.3 / 99.1, 192^3 155 / 169,
+    //     512x256x256 710 / 794
+    //   Smagorinsky cavities: 32^3 7.3 / 5.0, 64^3 9.9 / 7.7, 96^3 27.6 / 19.1, 128^3
+    //     46.0 / 42.0, 160^3 99.5 / 89.1, 192^3 150 / 153, 256^3 340 / 358, 512^3 2596 / 2863
+    // Small lattices leave multiprocessors without a march.  One border for both at
+    // 2^20 cells, the right one without Smagorinsky: with it the one-cell kernel
+    // would still be 9 to 11 % faster up to about 6 M cells.
     static bool w2_default(int storage, int q, bool flags, bool gray, std::size_t cells) {
         return storage == kStoreF16S && q == 19 && flags && !gray && cells >= (std::size_t{1} << 20);
     }
@@ -321,8 +325,10 @@ struct cfdx_lbm {
     // 3390, 256^3 445 / 431, D3Q27 192^3 283 / 270, FP64 cavity 160^3 246 / 222,
     // periodic FP16 192^3 123 / 114; reverse sweeps of a gray channel D3Q27 FP16
     // 160^3 (32 steps) 15.7 / 14.5 ms, D3Q19 FP16 128^3 17.1 / 15.9, FP32 17.7 / 17.5
-    // (32768 to 131072 cells: within 2 %).  The FP16 pair and one-cell kernels
-    // with flags, bound by issue slots, lose 1 to 2 % and have none.  None either
+    // (32768 to 131072 cells: within 2 %).  k_step_w2 and the FP16 one-cell
+    // kernel, bound by issue slots, lose 1 to 2 % and have none; k_step_h2 has it with
+    // flags, too, where it is chosen by hand (256^3 LES cavity 450 / 416, 160^3 channel
+    // 105 / 97, 256x128x128 sphere pack 114 / 110).  None either
     // for lattices that stay in L2 (`resident` bytes: the live lattice is read
     // again and again, frames are read once each), nor where the planes that a
     // pass keeps in L2 between a slot's neighbours would not fit beside it.
