@@ -539,6 +539,12 @@ def target_summary(line, variants):
 
 
 # ----------------------------------------------------------- reference (CPU)
+def reference_missing(path):
+    """Why the part of the reference's CPU build at `path` cannot be timed here, or None: it is made
+    from the reference's sources (make -C oracle ref), which a machine need not have."""
+    return None if os.path.exists(path) else f"the reference's CPU build has no {os.path.basename(path)} here"
+
+
 def cpu_reference_sample(n, warmup, steps, threads=0):
     """The reference's CPU path on the closest feature set: EsotericPullSolver<D3Q19>
     BGK + Smagorinsky with the cavity's walls and lid as a static solid mask
@@ -559,6 +565,10 @@ CPU_SAMPLE_SECONDS = 20.0
 
 def cpu_solid_baseline(max_seconds=CPU_SAMPLE_SECONDS):
     """cpu_baseline of the cavity line: the shared sample, timed steps sized to about max_seconds."""
+    from oracle import oracle as O
+
+    if why := reference_missing(O.REF_FAST_SO):
+        return {"unavailable": why}
     n = SOLID_SAMPLE_N
     _, per_step, _ = cpu_reference_sample(n, 0, 1)
     steps = max(2, int(max_seconds / max(per_step, 1e-3)))
@@ -596,6 +606,10 @@ def cpu_inplace_sample(n, seconds=CPU_SAMPLE_SECONDS, warmup=10):
 
 def cpu_inplace_baselines():
     """cfd-bench in-place at the plain-method size (64^3) and at 512^3, one sample length each."""
+    from oracle import oracle as O
+
+    if why := reference_missing(O.REF_CLI):
+        return {"unavailable": why}
     out = {}
     for n in (64, 512):
         r = cpu_inplace_sample(n)
@@ -805,7 +819,12 @@ def run_reference_arm(args, rank, world):
     """The reference's own CPU path for the cavity workload on the host cores: the same lattice as
     cpu_baseline (SOLID_SAMPLE_N^3, 3-pass solid step, Smagorinsky), smaller only when W + K steps of
     it would not end within about two minutes."""
+    from oracle import oracle as O
+
     if rank != 0:
+        return 0
+    if why := reference_missing(O.REF_FAST_SO):
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return 0
     _, per_step, _ = cpu_reference_sample(SOLID_SAMPLE_N, 0, 1)
     budget = 110.0
