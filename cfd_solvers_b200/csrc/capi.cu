@@ -232,8 +232,8 @@ struct cfdx_lbm {
     // longer tail: about one block's march on top of its share of the work, at
     // five resident blocks per SM.  B200, us per step at 4 / 3 / 2 / 1 planes:
     // LES cavities 512^3 2395 / 2404 / 2437 / 2758, 256^3 329 / 330 / 325 / -, 128^3
-    // 48.9 / 46.7 / 44.4 / 44.2 (short bursts; 46 at the rule's 2 under load), 64^3 24.3 / 16.2 / 13.5 / 9.8; sphere packs
-    // 512x256x256 686 / 695 / 716 / -, 100x90x80 25.4 / 24.6 / 23.1 / 22.4.
+    // 48.9 / 46.7 / 44.4 / 44.2 (short bursts; 46 at the rule's 2 under load), 64^3 24.3 /
+    // 16.2 / 13.5 / 9.8; sphere packs 512x256x256 686 / 695 / 716 / -, 100x90x80 25.4 / 24.6 / 23.1 / 22.4.
     std::uint32_t auto_planes() const {
         const std::size_t across = (cfg.nx / 2U + 31U) / 32U * ((cfg.ny + 3U) / 4U);
         const std::size_t resident = 5U * static_cast<std::size_t>(std::max(sms, 1));
@@ -1856,7 +1856,7 @@ void adjoint_buffer(void** p, std::size_t* have, std::size_t bytes, const char* 
 bool two_level(std::uint64_t sub, std::uint64_t len) { return sub >= 2U && sub < len; }
 
 // Recompute frames of the reverse sweep.  One level: interval - 1 frames,
-// the states inside a segment.  Two levels (sub-checkpoint interval m): the
+// the states inside a segment (the last segment's from the forward pass on).  Two levels (sub-checkpoint interval m): the
 // ceil(interval / m) - 1 sub-checkpoints of a segment, then the m - 1 states
 // inside one sub-segment.  The forward pass, and the first recompute pass of
 // two levels, use two of the frames as ping-pong buffers.

@@ -292,19 +292,21 @@ CFDX_API int cfdx_lbm_set_tau(cfdx_lbm* lbm, float tau);
  *
  * cfdx_lbm_adjoint_forward: runs `steps` steps from the current state like
  * cfdx_lbm_step, keeping a device copy of the lattice every `interval` steps
- * (ceil(steps/interval) copies, in the storage precision) plus the reverse
- * sweep's recompute frames (max(interval-1, 2) lattices with one level of
- * recompute; see cfdx_lbm_adjoint_set_subinterval).  It runs the out-of-place form of the
+ * counted from the last one (ceil(steps/interval) copies, in the storage
+ * precision; the first segment takes the remainder) plus the reverse sweep's
+ * recompute frames (max(interval-1, 2) lattices with one level of recompute; see
+ * cfdx_lbm_adjoint_set_subinterval), which hold the states of the last segment
+ * when it returns.  It runs the out-of-place form of the
  * step that the reverse sweep recomputes with, so the recomputed states equal
  * the forward's bit for bit; the final state equals cfdx_lbm_step(steps)'s to
  * within the last bit of the arithmetic type. */
 CFDX_API int cfdx_lbm_adjoint_forward(cfdx_lbm* lbm, uint64_t steps, uint32_t interval);
 
 /* Sub-checkpoint interval m of the reverse sweep for the following
- * cfdx_lbm_adjoint_forward calls: 0 (the default) recomputes each segment once
- * and holds its interval - 1 states; 2 <= m < interval recomputes it twice
- * (first every m-th state, then each sub-segment of m steps from its
- * sub-checkpoint) and holds ceil(interval/m) - 1 + max(m - 1, 2) frames
+ * cfdx_lbm_adjoint_forward calls: 0 (the default) recomputes each segment but
+ * the last once and holds its interval - 1 states; 2 <= m < interval recomputes
+ * it twice (first every m-th state, then each sub-segment of m steps from its
+ * sub-checkpoint; the last segment once) and holds ceil(interval/m) - 1 + max(m - 1, 2) frames
  * instead, e.g. 14 instead of 63 for interval 64 and m = 8.  The gradients are
  * bitwise the same.  1 is rejected (CFDX_ERR_INVALID). */
 CFDX_API int cfdx_lbm_adjoint_set_subinterval(cfdx_lbm* lbm, uint32_t subinterval);
@@ -314,10 +316,13 @@ CFDX_API int cfdx_lbm_adjoint_set_subinterval(cfdx_lbm* lbm, uint32_t subinterva
  * cfdx_lbm_macroscopic reports (u includes +a/2), all on `where` (host or
  * device).  Writes dJ/dn_s per cell (N doubles, 0 on walls; `grad_where`;
  * NULL skips) and dJ/dtau (*grad_tau, host; NULL skips).  Recomputes each
- * segment from its checkpoint; the lattice and its parameters must not have
+ * segment from its checkpoint, but takes the last one's states from where the
+ * forward pass left them; the lattice and its parameters must not have
  * changed since cfdx_lbm_adjoint_forward (else CFDX_ERR_INVALID).  FP32
  * adjoint arithmetic for FP32/FP16 storage, FP64 for FP64 storage; the
- * gradients are accumulated in FP64.  May be called again with another seed. */
+ * gradients are accumulated in FP64.  May be called again with another seed: a
+ * later sweep gives the same gradients, and recomputes the last segment as well
+ * (the first one used its frames) unless the pass is one segment of one level. */
 CFDX_API int cfdx_lbm_adjoint_backward(cfdx_lbm* lbm, const float* g_rho, const float* g_ux, const float* g_uy,
                                        const float* g_uz, int where, double* grad_ns, int grad_where,
                                        double* grad_tau);
