@@ -325,18 +325,22 @@ struct cfdx_lbm {
     // 3390, 256^3 445 / 431, D3Q27 192^3 283 / 270, FP64 cavity 160^3 246 / 222,
     // periodic FP16 192^3 123 / 114; reverse sweeps of a gray channel D3Q27 FP16
     // 160^3 (32 steps) 15.7 / 14.5 ms, D3Q19 FP16 128^3 17.1 / 15.9, FP32 17.7 / 17.5
-    // (32768 to 131072 cells: within 2 %).  k_step_w2 and the FP16 one-cell
+    // (32768 to 131072 cells: within 2 %).  FP64 lattices take half the distance, the
+    // same bytes: D3Q27 128^3 periodic, us per step without / 32768 / 65536, 139 / 139 /
+    // 143, 160^3 306 / 277 / 273.  k_step_w2 and the FP16 one-cell
     // kernel, bound by issue slots, lose 1 to 2 % and have none; k_step_h2 has it with
     // flags, too, where it is chosen by hand (256^3 LES cavity 450 / 416, 160^3 channel
     // 105 / 97, 256x128x128 sphere pack 114 / 110).  None either
-    // for lattices that stay in L2 (`resident` bytes: the live lattice is read
-    // again and again, frames are read once each), nor where the planes that a
+    // for lattices that L2 (126 MB) holds in good part (`resident` bytes: the live lattice is
+    // read again and again, frames are read once each; with / without, D3Q27 FP32 104 MB
+    // 37.2 / 33.4, 128 MB 47.5 / 45.6, 181 MB 62 / 62, D3Q19 FP64 cavity 103 MB 43.1 / 41.3,
+    // 134 MB 49.9 / 53.9, 500x400x4 122 MB 29.5 / 21.5), nor where the planes that a
     // pass keeps in L2 between a slot's neighbours would not fit beside it.
-    static constexpr std::size_t kResidentLattice = std::size_t{96} << 20, kStreamedLattice = std::size_t{24} << 20;
+    static constexpr std::size_t kResidentLattice = std::size_t{126} << 20, kStreamedLattice = std::size_t{24} << 20;
     std::uint32_t prefetch_distance(std::size_t elem_bytes, std::size_t resident) const {
         const std::size_t per_cell = static_cast<std::size_t>(key.q) * elem_bytes;
         const bool off = per_cell * N < resident || per_cell * cfg.nx * cfg.ny > (std::size_t{32} << 20);
-        return off ? 0U : 65536U;
+        return off ? 0U : (elem_bytes == 8U ? 32768U : 65536U);
     }
     LbmArgs args() const {
         LbmArgs a = args_at(f, storage_bytes(key.storage), static_cast<int>(t & 1U));

@@ -355,8 +355,12 @@ __global__ void __launch_bounds__(128, adjoint_min_blocks<L, S>()) k_adjoint_ste
     const u32 x = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 y = blockIdx.y * blockDim.y + threadIdx.y;
     const u32 z = blockIdx.z, y0 = blockIdx.y * blockDim.y, rows = min(blockDim.y, f.ny - y0);
-    prefetch_rows<L, typename S::T>(f, z * f.ny + y0, rows);
-    prefetch_rows<L, typename LS::T>(A.l, z * f.ny + y0, rows);
+    // Which of its two lattices to ask for, measured (us per step of a periodic sweep at interval 12
+    // without / frames / adjoint lattice / both): D3Q27 FP64 128^3 473 / 492 / 492 / 505 (160^3 1075 /
+    // 1067 / 1088 / 1088), D3Q27 FP32 128^3 300 / 304 / 304 / 305, 160^3 636 / 612 / 603 / 591,
+    // 97x65x66 74 / 76 / 75 / 78; D3Q27 FP16 160^3 615 / - / 528 / 519.
+    if constexpr (sizeof(typename S::T) == 2) prefetch_rows<L, typename S::T>(f, z * f.ny + y0, rows);
+    if constexpr (sizeof(typename LS::T) == 4) prefetch_rows<L, typename LS::T>(A.l, z * f.ny + y0, rows);
     double g_tau = 0.0;
     if (x < f.nx && y < f.ny) {
         const u32 n = (z * f.ny + y) * f.nx + x;

@@ -14,13 +14,14 @@ from test_gpu_slabs import sliced, whole
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("lattice, storage, shape", [("d3q19", "fp32", (131, 97, 130)), ("d3q27", "fp32", (101, 100, 96)),
-                                                     ("d3q19", "fp64", (90, 97, 81)), ("d3q27", "fp64", (77, 78, 79))])
+@pytest.mark.parametrize("lattice, storage, shape", [("d3q19", "fp32", (131, 97, 150)), ("d3q27", "fp32", (133, 100, 96)),
+                                                     ("d3q19", "fp64", (90, 97, 105)), ("d3q27", "fp64", (77, 78, 105)),
+                                                     ("d3q19", "fp32", (33, 250, 230))])  # rows too short for it
 def test_prefetch_equals_slabs(engine, lattice, storage, shape):
     cs = engine
     nx, ny, nz = shape
     q, es = {"d3q19": 19, "d3q27": 27}[lattice], {"fp32": 4, "fp64": 8}[storage]
-    assert q * es * nx * ny * nz > 96 << 20  # the whole lattice takes the prefetch, thirds of it do not
+    assert q * es * nx * ny * nz > 126 << 20  # the whole lattice takes the prefetch, thirds of it do not
     rng = np.random.default_rng(1)
     flags = (rng.uniform(size=(nz, ny, nx)) < 0.05).astype(np.uint8).reshape(-1)
     cfg = cs.InPlaceLbmConfig(nx=nx, ny=ny, nz=nz, tau=0.6, lattice=lattice, storage=storage, collision="trt")
@@ -31,9 +32,10 @@ def test_prefetch_equals_slabs(engine, lattice, storage, shape):
         assert np.array_equal(u, v)
 
 
-@pytest.mark.parametrize("shape", [(140, 139, 141), (1002, 60, 50)])
+@pytest.mark.parametrize("shape", [(140, 139, 190), (1002, 60, 62)])
 def test_prefetch_in_the_two_cell_kernel(engine, shape):
     cs = engine
+    assert 38 * np.prod(shape) > 126 << 20
     out = []
     for variant in (0, 1):
         with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=shape[0], ny=shape[1], nz=shape[2], tau=0.6,
@@ -48,7 +50,7 @@ def test_prefetch_in_the_two_cell_kernel(engine, shape):
 @pytest.mark.parametrize("lattice, storage", [("d3q19", "fp32"), ("d3q27", "fp16s")])
 def test_prefetch_in_the_reverse_sweep(engine, lattice, storage):
     cs = engine
-    nx, ny, nz = 121, 75, 62
+    nx, ny, nz = 131, 75, 62  # frames of 8 bytes past a multiple of 16, rows of more than 512 bytes
     n = nx * ny * nz
     rng = np.random.default_rng(2)
     ns = rng.uniform(0, 0.2, n).astype(np.float32)
