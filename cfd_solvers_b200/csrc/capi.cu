@@ -234,17 +234,19 @@ struct cfdx_lbm {
     // LES cavities 512^3 2395 / 2404 / 2437 / 2758, 256^3 329 / 330 / 325 / -, 128^3
     // 48.9 / 46.7 / 44.4 / 44.2 (short bursts; 46 at the rule's 2 under load), 64^3 24.3 /
     // 16.2 / 13.5 / 9.8; sphere packs 512x256x256 686 / 695 / 716 / -, 100x90x80 25.4 / 24.6 / 23.1 / 22.4.
+    // Where solids are scattered a march's start costs more than that (1 % single
+    // solid cells, 1000x100x100 247 / 250 / 256 / 299, 160^3 115 / 118 / 120 / 136, 128^3 52.5 /
+    // 52.8 / 52.8 / 54.4, 300x60x60 32.0 / 30.3 / 30.3 / 30.2), so a shorter march is taken only
+    // where the estimate expects 7 % from it; cavities between lose up to 3 %.
     std::uint32_t auto_planes() const {
         const std::size_t across = (cfg.nx / 2U + 31U) / 32U * ((cfg.ny + 3U) / 4U);
         const std::size_t resident = 5U * static_cast<std::size_t>(std::max(sms, 1));
         constexpr std::size_t march[5] = {0U, 1152U, 2035U, 3010U, 4000U};
+        const auto cost = [&](std::uint32_t k) { return (across * ((cfg.nz + k - 1U) / k) + resident) * march[k]; };
         std::uint32_t best = 4U;
-        for (std::uint32_t p = 3U; p >= 1U; --p) {
-            const auto cost = [&](std::uint32_t k) {
-                return (across * ((cfg.nz + k - 1U) / k) + resident) * march[k];
-            };
+        for (std::uint32_t p = 3U; p >= 1U; --p)
             if (cost(p) < cost(best)) best = p;
-        }
+        if (cost(best) * 100U > cost(4U) * 93U) best = 4U;
         return best;
     }
     // Automatic choice between the one-cell and the paired-cell kernel, from
