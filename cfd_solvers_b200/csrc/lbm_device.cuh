@@ -1450,26 +1450,42 @@ __device__ __forceinline__ void block_combine(double (&acc)[kReduceFields]) {
 }
 
 // Combines `blocks` rows of partial sums; thread 0 of the block gets the result.
+// FRESH: they were written by other blocks of this kernel, so loads go past L1.
+template <bool FRESH>
 __device__ __forceinline__ void combine_partials(const double* partials, int blocks, double (&acc)[kReduceFields]) {
 #pragma unroll
     for (int k = 0; k < kReduceFields; ++k) acc[k] = 0.0;
     for (int b = threadIdx.y * blockDim.x + threadIdx.x; b < blocks; b += kReduceThreads)
 #pragma unroll
         for (int k = 0; k < kReduceFields; ++k) {
-            const double v = __ldcg(partials + static_cast<std::size_t>(b) * kReduceFields + k);
+            const double* p = partials + static_cast<std::size_t>(b) * kReduceFields + k;
+            const double v = FRESH ? __ldcg(p) : *p;
             acc[k] = k == 5 ? fmax(acc[k], v) : acc[k] + v;
         }
     block_combine(acc);
 }
 
+// Resident blocks per SM (0: as many as the registers allow).  The grid of
+// cfdx_lbm_reduce has four blocks per SM, and they run in one wave at 64 registers,
+// where the forms that ask for four do not spill.  Left to itself the compiler gave
+// walled D3Q19 80 registers (three blocks, so two waves) and the open FP64 form 48
+// (too few for its loads in flight): one call, us (B200), 512x512x48 D3Q19 FP32 cavity
+// 306 / 202, FP16 305 / 216, D3Q27 FP64 periodic 587 / 409.  Walled D3Q27 and walled FP64
+// forms would spill at 64 registers and run at three and two blocks.
+template <class L, class S, bool FLAGS, bool FUSED> constexpr int reduce_min_blocks() {
+    if (!FLAGS) return 4;
+    return FUSED && L::Q == 19 && sizeof(typename S::T) != 8 ? 4 : 0;
+}
+
 template <class L, class S, bool FLAGS, bool FUSED>
-__global__ void __launch_bounds__(kReduceThreads) k_reduce(const __grid_constant__ LbmArgs a, double* partials,
+__global__ void __launch_bounds__(kReduceThreads, reduce_min_blocks<L, S, FLAGS, FUSED>()) k_reduce(const __grid_constant__ LbmArgs a, double* partials,
                                                            unsigned* done, double* out) {
     using R = typename S::R;
     dependent_begin();
     double acc[kReduceFields] = {0, 0, 0, 0, 0, 0, 0};
     const u32 rows = a.ny * a.nz;
-    for (u32 row = blockIdx.x * blockDim.y + threadIdx.y; row < rows; row += gridDim.x * blockDim.y) {
+    const u32 across = FUSED ? blockDim.y : 1U, first_row = FUSED ? blockIdx.x * across + threadIdx.y : blockIdx.x;
+    for (u32 row = first_row; row < rows; row += gridDim.x * across) {
         const u32 y = row % a.ny, z = row / a.ny;
         for (u32 x = threadIdx.x; x < a.nx; x += blockDim.x) {
             const u32 n = row * a.nx + x;
@@ -1511,7 +1527,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const __grid_constant
         __syncthreads();
         if (!last) return;
         __threadfence();
-        combine_partials(partials, static_cast<int>(gridDim.x), acc);
+        combine_partials<true>(partials, static_cast<int>(gridDim.x), acc);
         if (first) {
 #pragma unroll
             for (int k = 0; k < kReduceFields; ++k) out[k] = acc[k];
@@ -1523,7 +1539,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce(const __grid_constant
 static __global__ void __launch_bounds__(kReduceThreads) k_reduce_final(const double* partials, int blocks,
                                                                         double* out) {
     double acc[kReduceFields];
-    combine_partials(partials, blocks, acc);
+    combine_partials<false>(partials, blocks, acc);
     if (threadIdx.x == 0)
 #pragma unroll
         for (int k = 0; k < kReduceFields; ++k) out[k] = acc[k];

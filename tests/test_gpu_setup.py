@@ -203,3 +203,35 @@ def test_an_allocation_that_fails_leaves_no_error_behind(engine):
         s.initialize_uniform()
         s.step(2)
         assert s.reduce()["nonfinite"] == 0
+
+
+@pytest.mark.parametrize("lattice, storage, walls, ratio", [("d3q19", "fp32", True, 1.45), ("d3q27", "fp64", False, 1.25)])
+def test_sums_run_at_about_the_field_reads_rate(engine, lattice, storage, walls, ratio):
+    """The sums and the field read load the same populations.  A reduction whose blocks need a second
+    wave (too many registers) or whose loads wait in line (too few) takes 1.66 and 1.44 times as
+    long as the read here; in one wave 1.1 and 0.96, the host's share of a call included."""
+    import time
+
+    import torch
+
+    cs = engine
+    nx, ny, nz = 512, 512, 48
+    with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=nx, ny=ny, nz=nz, lattice=lattice, storage=storage)) as s:
+        if walls:
+            s.set_flags(cs.cavity_flags(nx, ny, nz))
+        s.initialize_taylor_green(0.03)
+
+        def best(call, n=10):
+            call()
+            times = []
+            for _ in range(6):
+                torch.cuda.synchronize()
+                t = time.perf_counter()
+                for _ in range(n):
+                    call()
+                torch.cuda.synchronize()
+                times.append((time.perf_counter() - t) / n)
+            return min(times)
+
+        read, sums = best(s.refresh_device_macroscopic), best(s.reduce)
+        assert sums < ratio * read, (sums, read)
