@@ -1077,8 +1077,8 @@ __device__ __forceinline__ void collide_scaled(const LbmArgs& a, u32 n, V* h) {
 // 12 blocks (40 registers) beat 10 once the wall path stopped branching (LES
 // cavity FP16 48.4 vs 46.9, FP32 40.6 vs 40.0; sphere pack within 0.5 %);
 // D3Q27 FP16 runs at 8 blocks (64 registers), where it does not spill: periodic
-// BGK 128^3 49.5 us against 54.6 at 10, 256x128x128 sphere pack 120.4 against
-// 123.2, 256^3 LES cavity 476 against 478.
+// BGK 128^3 53.0 us against 59.2 at 10, 256x128x128 sphere pack 123 against
+// 134, 256^3 LES cavity 508 against 522 (under load).
 // FP64 storage keeps its full register set.  The macros exist for tuning builds.
 #ifndef CFDX_STEP_MIN_BLOCKS_Q19
 #define CFDX_STEP_MIN_BLOCKS_Q19 12
