@@ -18,6 +18,7 @@
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "halo.h"
@@ -464,8 +465,8 @@ struct cfdx_lbm {
                   (variant == 0 && w2_default(key.storage, key.q, key.flags, key.gray, N))) &&
                  w2_eligible();
         key.w2_pipe = variant != 4;
-        key.paired = !key.w2 && (variant == 2 || (variant == 0 && paired_eligible() &&
-                                                  paired_default(key.storage, key.q, key.flags)));
+        key.paired = !key.w2 && paired_eligible() &&
+                     (variant == 2 || (variant == 0 && paired_default(key.storage, key.q, key.flags)));
     }
     dim3 step_block() const {
         if (key.w2) {
@@ -1645,24 +1646,24 @@ CFDX_API int cfdx_lbm_set_launch_shape(cfdx_lbm* h, int bx, int by, int variant)
         checked(h);
         require(variant >= 0 && variant <= 4,
                 "step kernel variant must be 0 (auto), 1 (one cell), 2 (paired) or 3 / 4 (wall-aware FP16 pairs)");
-        if (bx == 0 && by == 0) {
-            h->shape = LaunchShape{};
-        } else {
-            require(bx > 0 && by > 0 && bx * by <= 128 && (bx * by) % 32 == 0,
+        LaunchShape shape{};
+        if (bx != 0 || by != 0) {
+            require(bx > 0 && by > 0 && bx <= 128 && by <= 128 && bx * by <= 128 && (bx * by) % 32 == 0,
                     "block shape must have bx*by a multiple of 32 and at most 128");
-            h->shape = LaunchShape{bx, by};
+            shape = LaunchShape{bx, by};
         }
+        // A refused call leaves the handle as it was: the next call that chooses the kernel
+        // again must not find a variant that the lattice cannot take.
+        const LaunchShape before = std::exchange(h->shape, shape);
+        const bool fits = variant == 2 ? h->paired_eligible() : (variant < 3 || h->w2_eligible());
+        if (!fits) h->shape = before;
+        require(fits || variant != 2,
+                "the paired-cell kernel needs FP32/FP16 storage, an even nx, q*cells < 2^32 and block_x a "
+                "multiple of 32");
+        require(fits, "the wall-aware paired kernel needs FP16 storage, an even nx, q*cells < 2^32 and 128-thread "
+                      "blocks");
         h->variant = variant;
         h->key.cells_per_thread = 1;
-        if (variant == 2)
-            require(h->paired_eligible(),
-                    "the paired-cell kernel needs FP32/FP16 storage, an even nx, q*cells < 2^32 and block_x a "
-                    "multiple of 32");
-        if (variant == 3 || variant == 4)
-            require(h->w2_eligible(),
-                    "the wall-aware paired kernel needs FP16 storage, an even nx, q*cells < 2^32 and 128-thread "
-                    "blocks");
-
         h->choose_variant();
         refresh_near_list(h, false);
     });

@@ -66,6 +66,42 @@ def test_paired_variant_requires_even_nx(engine):
         s.step(3)
 
 
+@pytest.mark.parametrize("storage, shape", [("fp16s", (17, 6, 5)), ("fp32", (17, 6, 5)), ("fp64", (16, 6, 5)),
+                                            ("fp16s", (16, 6, 5)), ("fp32", (16, 6, 5))])
+def test_a_refused_launch_shape_leaves_the_handle_as_it_was(engine, storage, shape):
+    """Every setter that chooses the kernel again used to find the refused variant: an odd row in the
+    two-cell kernel.  Refused variants and shapes between setters change nothing."""
+    cs = engine
+    nx, ny, nz = shape
+    n = nx * ny * nz
+    rng = np.random.default_rng(4)
+    flags, ns = (rng.random(n) < 0.1).astype(np.uint8), rng.uniform(0, 0.2, n).astype(np.float32)
+    refused = [(0, 0, 5), (0, 0, -1), (48, 1, 0), (256, 1, 0), (64, 0, 0)]
+    if nx % 2 or storage == "fp64":
+        refused += [(0, 0, 2), (32, 4, 2)]
+    else:
+        refused += [(16, 4, 2)]  # the two-cell kernels take whole warps along x
+    refused += [(0, 0, 3), (0, 0, 4)] if nx % 2 or storage != "fp16s" else [(32, 1, 3)]
+    out = []
+    for refuse in (False, True):
+        def tries(s):
+            for bx, by, variant in refused if refuse else []:
+                with pytest.raises(ValueError):
+                    s.set_launch_shape(bx, by, variant)
+
+        with cs.EsotericPullCudaSolver(cs.InPlaceLbmConfig(nx=nx, ny=ny, nz=nz, tau=0.6, storage=storage)) as s:
+            tries(s)
+            s.initialize_taylor_green(0.05)
+            s.step(2)
+            s.set_flags(flags)
+            s.step(2)
+            tries(s)
+            s.set_solid_fraction(ns)
+            s.step(3)
+            out.append(s.logical_populations())
+    assert np.array_equal(out[0], out[1])
+
+
 # The wall-aware FP16 pair kernel (variants 3 and 4) marches along z; plane
 # counts that do not divide nz leave a short last chunk, and rows of 256 cells
 # span more than one warp.  The pipelined form (variant 3) reads flags three
