@@ -121,3 +121,51 @@ def test_overlapping_launches_equal_separate_ones(engine, q, storage, variant, k
             out.append((seen, s.logical_populations()))
     assert out[0][0] == out[1][0]
     assert np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("q, storage, kind, variant", [(19, "fp32", "periodic", 0), (27, "fp64", "gray", 0),
+                                                       (19, "fp32", "cavity", 2), (19, "fp16s", "cavity", 3),
+                                                       (19, "fp16s", "periodic", 0), (19, "fp16s", "cavity", 2)])
+def test_steps_under_a_callers_capture(engine, q, storage, kind, variant):
+    """Dependent launches recorded by a caller's capture of the solver's stream: beside a fork to
+    another stream that joins again, a memset and a field read, a replay equals the same calls."""
+    import torch
+
+    cs = engine
+    out = []
+    for captured in (False, True):
+        with solver(cs, q, storage, kind, variant) as s:
+            s.refresh_device_macroscopic()  # allocates its fields
+            s.wait()
+            stream, side = torch.cuda.ExternalStream(s.stream()), torch.cuda.Stream()
+            buf = torch.zeros(1 << 14, device="cuda")
+            torch.cuda.synchronize()
+
+            def calls():
+                s.step(2)
+                side.wait_stream(stream)
+                with torch.cuda.stream(side):
+                    buf.add_(1.0)
+                stream.wait_stream(side)
+                s.step(2)
+                buf.zero_()
+                s.step(1)
+                s.refresh_device_macroscopic()
+                s.step(9)
+
+            with torch.cuda.stream(stream):
+                if captured:
+                    graph = torch.cuda.CUDAGraph()
+                    graph.capture_begin(capture_error_mode="thread_local")
+                    try:
+                        calls()
+                    finally:
+                        graph.capture_end()
+                    graph.replay()
+                    torch.cuda.synchronize()
+                    del graph
+                else:
+                    calls()
+            torch.cuda.synchronize()
+            out.append(s.logical_populations())
+    assert np.array_equal(out[0], out[1])
