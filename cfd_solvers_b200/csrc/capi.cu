@@ -328,7 +328,8 @@ struct cfdx_lbm {
     // 3390, 256^3 445 / 431, D3Q27 192^3 283 / 270, FP64 cavity 160^3 246 / 222,
     // periodic FP16 192^3 123 / 114; reverse sweeps of a gray channel D3Q27 FP16
     // 160^3 (32 steps) 15.7 / 14.5 ms, D3Q19 FP16 128^3 17.1 / 15.9, FP32 17.7 / 17.5
-    // (32768 to 131072 cells: within 2 %).  FP64 lattices take half the distance, the
+    // (32768 to 131072 cells: within 2 %; which lattices the reverse sweep asks for
+    // stands beside k_adjoint_step).  FP64 lattices take half the distance, the
     // same bytes: D3Q27 128^3 periodic, us per step without / 32768 / 65536, 139 / 139 /
     // 143, 160^3 306 / 277 / 273.  k_step_w2 and the FP16 one-cell
     // kernel, bound by issue slots, lose 1 to 2 % and have none; k_step_h2 has it with

@@ -1478,8 +1478,8 @@ template <class L, class S, bool FLAGS, bool FUSED> constexpr int reduce_min_blo
 }
 
 template <class L, class S, bool FLAGS, bool FUSED>
-__global__ void __launch_bounds__(kReduceThreads, reduce_min_blocks<L, S, FLAGS, FUSED>()) k_reduce(const __grid_constant__ LbmArgs a, double* partials,
-                                                           unsigned* done, double* out) {
+__global__ void __launch_bounds__(kReduceThreads, reduce_min_blocks<L, S, FLAGS, FUSED>())
+    k_reduce(const __grid_constant__ LbmArgs a, double* partials, unsigned* done, double* out) {
     using R = typename S::R;
     dependent_begin();
     double acc[kReduceFields] = {0, 0, 0, 0, 0, 0, 0};
