@@ -344,7 +344,9 @@ struct cfdx_lbm {
     std::uint32_t prefetch_distance(std::size_t elem_bytes, std::size_t resident) const {
         const std::size_t per_cell = static_cast<std::size_t>(key.q) * elem_bytes;
         const bool off = per_cell * N < resident || per_cell * cfg.nx * cfg.ny > (std::size_t{32} << 20);
-        return off ? 0U : (elem_bytes == 8U ? 32768U : 65536U);
+        if (off) return 0U;
+        const std::size_t two_planes = std::min<std::size_t>(2U * cfg.nx * cfg.ny, 65536U);
+        return elem_bytes == 8U ? std::max(32768U, static_cast<std::uint32_t>(two_planes)) : 65536U;
     }
     LbmArgs args() const {
         LbmArgs a = args_at(f, storage_bytes(key.storage), static_cast<int>(t & 1U));
