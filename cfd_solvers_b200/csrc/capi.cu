@@ -329,9 +329,11 @@ struct cfdx_lbm {
     // periodic FP16 192^3 123 / 114; reverse sweeps of a gray channel D3Q27 FP16
     // 160^3 (32 steps) 15.7 / 14.5 ms, D3Q19 FP16 128^3 17.1 / 15.9, FP32 17.7 / 17.5
     // (32768 to 131072 cells: within 2 %; which lattices the reverse sweep asks for
-    // stands beside k_adjoint_step).  FP64 lattices take half the distance, the
-    // same bytes: D3Q27 128^3 periodic, us per step without / 32768 / 65536, 139 / 139 /
-    // 143, 160^3 306 / 277 / 273.  k_step_w2 and the FP16 one-cell
+    // stands beside k_adjoint_step).  FP64 lattices run two
+    // planes ahead within 32768 and 65536 cells: less than one plane misses the rows of the
+    // next plane that a step reads, more is as many bytes as L2 has better use for (D3Q27
+    // periodic, us per step without / 32768 / 65536 / two planes: 128^3 139 / 138 / 141 / 138,
+    // 144x144x100 166 / 147 / 143 / 140, 194x262x31 124 / 118 / 108 / 108).  k_step_w2 and the FP16 one-cell
     // kernel, bound by issue slots, lose 1 to 2 % and have none; k_step_h2 has it with
     // flags, too, where it is chosen by hand (256^3 LES cavity 450 / 416, 160^3 channel
     // 105 / 97, 256x128x128 sphere pack 114 / 110).  None either
