@@ -341,11 +341,15 @@ struct cfdx_lbm {
     // read again and again, frames are read once each; with / without, D3Q27 FP32 104 MB
     // 37.2 / 33.4, 128 MB 47.5 / 45.6, 181 MB 62 / 62, D3Q19 FP64 cavity 103 MB 43.1 / 41.3,
     // 134 MB 49.9 / 53.9, 500x400x4 122 MB 29.5 / 21.5), nor where the planes that a
-    // pass keeps in L2 between a slot's neighbours would not fit beside it.
+    // pass keeps in L2 between a slot's neighbours would not fit beside it, nor where a
+    // block's rows make requests of under 512 bytes (FP32 periodic lattices of 4 M cells,
+    // with / without, us per step: D3Q19 33 cells wide 143 / 129, 40 122 / 117, 72 112 / 106, 128
+    // 99 / 99, 160 97 / 100; D3Q27 197 / 179, 170 / 165, 159 / 149, 137 / 137, 137 / 140).
     static constexpr std::size_t kResidentLattice = std::size_t{126} << 20, kStreamedLattice = std::size_t{24} << 20;
     std::uint32_t prefetch_distance(std::size_t elem_bytes, std::size_t resident) const {
         const std::size_t per_cell = static_cast<std::size_t>(key.q) * elem_bytes;
-        const bool off = per_cell * N < resident || per_cell * cfg.nx * cfg.ny > (std::size_t{32} << 20);
+        const bool off = per_cell * N < resident || per_cell * cfg.nx * cfg.ny > (std::size_t{32} << 20) ||
+                         elem_bytes * cfg.nx * block().y < 512U;
         if (off) return 0U;
         const std::size_t two_planes = std::min<std::size_t>(2U * cfg.nx * cfg.ny, 65536U);
         return elem_bytes == 8U ? std::max(32768U, static_cast<std::uint32_t>(two_planes)) : 65536U;

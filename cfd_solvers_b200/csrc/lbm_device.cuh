@@ -488,18 +488,13 @@ __device__ __forceinline__ void scatter(const LbmArgs& a, u32 n, const Nbr& o, c
 // Asks L2 for the populations that lie a.ahead cells after the rows of this
 // block (`rows` of them from row index `row` on), one bulk request per
 // direction from the first block of the rows, so every row is asked for once
-// (whole rows: a request per 128 cells slowed D3Q27 down; rows of less than
-// kPrefetchBytes together are not asked for: FP32 periodic lattices of 4 M cells
-// with / without, us per step, D3Q19 33 cells wide 143 / 129, 40 122 / 117, 72 112 /
-// 106, 128 99 / 99, 160 97 / 100; D3Q27 197 / 179, 170 / 165, 159 / 149, 137 / 137, 137 / 140).
-// The kernels hold their loads' latency with resident warps alone, and registers
-// limit those.
-constexpr u32 kPrefetchBytes = 512U;
+// (whole rows: a request per 128 cells slowed D3Q27 down).  The kernels hold
+// their loads' latency with resident warps alone, and registers limit those.
 template <class L, class T> __device__ __forceinline__ void prefetch_rows(const LbmArgs& a, u32 row, u32 rows) {
     const u32 d = threadIdx.y * blockDim.x + threadIdx.x;
-    const u32 cells = rows * a.nx;
-    if (a.ahead == 0U || blockIdx.x != 0U || d >= static_cast<u32>(L::Q) || cells * sizeof(T) < kPrefetchBytes) return;
+    if (a.ahead == 0U || blockIdx.x != 0U || d >= static_cast<u32>(L::Q)) return;
     const unsigned long long m = static_cast<unsigned long long>(row) * a.nx + a.ahead;
+    const u32 cells = rows * a.nx;
     if (m + cells + 16U > a.N) return; // whole 16-byte units inside the direction
     // the request wants a 16-byte aligned address and size; the lattice itself may start at any
     // element (the adjoint's frames lie one after the other)
